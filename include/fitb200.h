@@ -197,15 +197,18 @@ int fitb_spectral_dt(fitb_handle* h, double safety, int32_t max_iter, double tol
  * round-off; they halve the coefficient reads (96 -> 72 bytes per cell and
  * step in float32).  No counterpart in the reference, which stores the
  * coefficients in the field dtype (fit_td.py:468-479).  Valid before or
- * after fitb_set_coeffs; FITB_ERR_STATE when the handle does not use the
- * stream kernels. */
+ * after fitb_set_coeffs; FITB_ERR_STATE when the handle was configured to a
+ * form without them (they are in the stream and vec kernels, float16 also in
+ * the float32 slab step, and in the direct kernels of a handle nobody
+ * configured). */
 #define FITB_COEF_NATIVE 0
 #define FITB_COEF_F16 1
 #define FITB_COEF_BF16 2
 int fitb_set_coeff_storage(fitb_handle* h, int32_t kind);
 /* Stencil form of the handle (no counterpart in the reference, whose kernels
- * are fixed): kind FITB_STENCIL_SIMPLE / STREAM / BULK / VEC / FUSED, a
- * variant of that form (vec 0-3; fused 0-6 the register / cp.async forms,
+ * are fixed; a handle nobody configured runs the direct kernels of
+ * FITB_STENCIL_SIMPLE): kind FITB_STENCIL_SIMPLE / STREAM / BULK / VEC / FUSED,
+ * a variant of that form (vec 0-3; fused 0-6 the register / cp.async forms,
  * fused 7-15 the TMA tile form with its CPML slab passes, tile shapes of
  * 2-16 rows x 32 cells and 3-5 ring stages; fused 16-25 the slab step, the
  * TMA tile march with the CPML inside it, tiles of 4, 2, 3, 4, 3, 2, 8, 6,

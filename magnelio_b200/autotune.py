@@ -26,6 +26,7 @@ from magnelio_b200._lib import FitbError
 
 # (kind, variant, i planes per CTA; 0 = the form's own plan)
 DEFAULT_CANDIDATES = (
+    ("simple", 0, 0),
     ("stream", 0, 0),
     ("stream", 1, 0),
     ("stream", 2, 0),
@@ -54,7 +55,7 @@ DEFAULT_CANDIDATES = (
     ("fused", 25, 0),
     ("bulk", 0, 0),
 )
-CANDIDATE_SET = 6  # bump when the candidates change: cached results of another set are not reused
+CANDIDATE_SET = 7  # bump when the candidates change: cached results of another set are not reused
 
 
 @dataclass

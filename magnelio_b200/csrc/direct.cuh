@@ -1,0 +1,54 @@
+// Arguments and launchers of the direct stencil kernels (stencil.cu): one
+// cell per thread, any number of field sets.
+#pragma once
+#include "fitb_common.cuh"
+
+namespace fitb {
+
+// What the direct kernels take beside StencilArgs (stencil.cu): the launcher
+// fills the division and the slab bounds, the caller the planes per thread,
+// the one-edge lumped ports that step inside the E kernel (their cell and
+// component; `ports` the device table in the same order) and the step counter
+// the H kernel advances (null: not advanced there).
+constexpr int kDirectLumped = 16;
+// The CPML faces of one axis: [0] the layers 0 .. n[0] - 1, [1] the layers
+// lo1 .. lo1 + n[1] - 1 (lo1 = INT_MAX: none).  Entry of cell (i, j, k):
+// s0 i + s1 j + k with the layer in place of the axis coordinate.  psi, air:
+// the first of the side's (E or H) two auxiliaries, the second `slab` entries
+// further on, a field set's `set` entries apart; air null without PEC masks.
+struct AxisSlabs {
+    int lo1;
+    int n[2], s0[2], s1[2];
+    unsigned slab[2];
+    size_t set[2];
+    void* psi[2];
+    const void* bcc[2];
+    const unsigned char* air[2];
+};
+struct DirectDiv {
+    unsigned m;
+    int s;
+};
+struct DirectArgs {
+    int np;
+    // vectors of a row: n_low in the near z slab, n_mid clear of both, n_edge
+    // = all but the n_mid; a plane's first mid_threads threads take the clear ones
+    int n_low, n_mid, n_edge;
+    unsigned mid_threads;
+    DirectDiv mid_div, edge_div;
+    AxisSlabs ax[3];
+    int n_lumped;
+    int4 lumped[kDirectLumped];
+    const LumpedDev* ports;
+    PortsArgs pa;
+    long long* advance;
+};
+// which: 0 = E update, 1 = H update
+template <typename T>
+void launch_direct_half(const StencilArgs<T>& a, const DirectArgs& d, int which, cudaStream_t s);
+// flags[side] (zeroed by the caller): bit 0 set when alpha is not (beta != 0),
+// bit 1 when it is not 1 everywhere.
+template <typename T>
+void launch_unit_alpha(const StencilArgs<T>& a, int* flags, cudaStream_t s);
+
+}  // namespace fitb

@@ -25,7 +25,7 @@
 #include <vector>
 
 #include "../../include/fitb200.h"
-#include "fitb_common.cuh"
+#include "direct.cuh"
 
 namespace fitb {
 
@@ -174,6 +174,7 @@ struct PlaneWaveHost {
 struct ModalHost {
     ModalDev dev{};
     std::vector<long long> port_e_host;  // E offsets the port writes
+    std::vector<long long> int_e_host;   // and those of the interior plane it reads
     int n_modes = 0;
     DevBuf port_e, int_e, port_h, me_port, me_int, mh_port, eprof, vprof, hprof;
     DevBuf comp_r, comp_live;
@@ -263,9 +264,9 @@ struct Handle {
     std::vector<std::unique_ptr<BandHost>> band;  // band-subspace DTBC ports
     DevBuf d_band;
     DevBuf d_lumped, d_modal, d_dft;
-    int dft_stage_blocks = 0, dft_flush_blocks = 0;
-    size_t dft_flush_smem = 0;
-    DevBuf ticket;  // CTA completion counter of the merged flush launch
+    int dft_blocks = 0;
+    size_t dft_smem = 0;
+    DevBuf ticket;  // CTA completion counter of the monitor launch
     int launches_per_step = 0;
     bool port_tables_dirty = true;
     DevBuf step;          // long long
@@ -281,7 +282,22 @@ struct Handle {
     int chunk = 16;
     bool graphs_valid = false;
     long long launches = 0;
-    int ichunk = 16;
+    int direct_np = 0;  // planes per thread of the direct kernels (0: their own choice)
+    // The stencil form is the engine's own choice, the direct kernels (no
+    // FITB_STENCIL, no fitb_configure_stencil): the fastest form at every
+    // size, batch and precision measured, from 8 us against the stream
+    // kernels' 41 us per step at 10 thousand cells to 1.82 ms against 2.56 ms
+    // (slab step: 2.25 ms) at 105 million.  It takes the compact coefficient
+    // storage, which an explicitly configured "simple" form refuses.
+    bool auto_form = false;
+    // alpha follows from beta (StencilArgs::unit_alpha) in the coefficients
+    // as they are stored
+    int unit_alpha = 0;
+    float a0[2] = {};
+    DevBuf scan;  // flags of the coefficient scan
+    // lumped ports that step inside the direct E kernel (all or none)
+    bool lumped_in_E = false;
+    int4 lumped_cell[kDirectLumped] = {};
     // Bulk-copy pipelined stencil (single field set); status word of its
     // bounded waits.
     BulkPlan plan{};
@@ -425,7 +441,7 @@ size_t device_bytes(const Handle& H) {
     size_t n = 0;
     for (const DevBuf* d : {&H.e, &H.h, &H.e2, &H.h2, &H.aE, &H.bE, &H.aH, &H.bH, &H.meps, &H.mmu, &H.staging,
                             &H.fix_cells, &H.d_lumped, &H.d_modal, &H.d_dft, &H.ticket, &H.step, &H.recV, &H.recI,
-                            &H.absmax, &H.energy_partials, &H.energy_out, &H.status})
+                            &H.absmax, &H.energy_partials, &H.energy_out, &H.status, &H.scan})
         n += d->bytes;
     for (const auto& q : H.cq) n += q.bytes;
     for (const auto& f : H.faces) n += f->psi.bytes + f->psi2.bytes + f->air.bytes + f->bcc.bytes;
@@ -566,6 +582,34 @@ void build_fix_cells(Handle& H) {
 
 void build_slab_units(Handle& H);
 
+// The lumped ports may step inside the direct E kernel when each has one edge
+// of its own and nothing else touches that edge between the E update and the
+// ports: no plane wave, ADE or band port on the E side, and no modal port that
+// writes or reads the edge.
+void find_lumped_in_E(Handle& H) {
+    H.lumped_in_E = false;
+    if (H.lumped.empty() || (int)H.lumped.size() > kDirectLumped) return;
+    if (!H.pws.empty() || H.disp[0].present() || !H.band.empty()) return;
+    std::vector<long long> own;
+    for (auto& lp : H.lumped) {
+        if (lp->off_host.size() != 1) return;
+        own.push_back(lp->off_host[0]);
+    }
+    std::vector<long long> used = own;
+    std::sort(used.begin(), used.end());
+    if (std::adjacent_find(used.begin(), used.end()) != used.end()) return;
+    for (auto& mp : H.modal)
+        for (const std::vector<long long>* v : {&mp->port_e_host, &mp->int_e_host})
+            for (long long o : *v)
+                if (std::binary_search(used.begin(), used.end(), o)) return;
+    for (size_t q = 0; q < own.size(); ++q) {
+        const long long r = own[q] % H.g.vol, rr = r % H.g.si;
+        H.lumped_cell[q] = make_int4((int)(r / H.g.si) - 2, (int)(rr / H.g.sj), (int)(rr % H.g.sj),
+                                     (int)(own[q] / H.g.vol));
+    }
+    H.lumped_in_E = true;
+}
+
 void refresh_port_tables(Handle& H) {
     if (!H.port_tables_dirty) return;
     // the tables below are re-allocated: no launch may still read the old ones
@@ -573,6 +617,7 @@ void refresh_port_tables(Handle& H) {
     std::vector<LumpedDev> ld;
     for (auto& lp : H.lumped) ld.push_back(lp->dev);
     upload(H.d_lumped, ld);
+    find_lumped_in_E(H);
     std::vector<ModalDev> md;
     for (auto& mp : H.modal) {
         ModalDev d = mp->dev;
@@ -603,29 +648,23 @@ void refresh_port_tables(Handle& H) {
     upload(H.d_band, bd);
     // monitors: block ranges of the merged stage / flush launches
     std::vector<DftDev> dd;
-    int sb = 0, fb = 0;
+    int sb = 0;
     size_t smem = 0;
     for (auto& m : H.dft) {
         DftDev d = m->dev;
         d.sblk0 = sb;
-        d.sblk = dft_blocks((long long)d.ncomp * d.ncell);
-        d.fblk0 = fb;
-        d.fblk = dft_blocks((long long)H.B * d.ncomp * d.ncell);
+        d.sblk = fitb::dft_blocks((long long)d.ncomp * d.ncell);
         sb += d.sblk;
-        fb += d.fblk;
         smem = std::max(smem, (size_t)d.K * 2 * d.nf * sizeof(float2));
         m->dev.sblk0 = d.sblk0;
         m->dev.sblk = d.sblk;
-        m->dev.fblk0 = d.fblk0;
-        m->dev.fblk = d.fblk;
         dd.push_back(d);
     }
     upload(H.d_dft, dd);
     if (H.stencil_mode == kModeFused) build_fix_cells(H);
     if (H.stencil_mode == kModeFused && is_slab_variant(H.fused_variant)) build_slab_units(H);
-    H.dft_stage_blocks = sb;
-    H.dft_flush_blocks = fb;
-    H.dft_flush_smem = smem;
+    H.dft_blocks = sb;
+    H.dft_smem = smem;
     H.port_tables_dirty = false;
 }
 
@@ -645,11 +684,15 @@ StencilArgs<T> stencil_args(Handle& H) {
     a.nfaces = (int)H.faces.size();
     for (int q = 0; q < a.nfaces; ++q) {
         a.f[q] = H.faces[q]->dev;
+        a.f[q].masked = H.faces[q]->pec ? 1 : 0;
         if (H.cur) std::swap(a.f[q].psi, a.f[q].psi_next);
     }
-    a.ichunk = H.ichunk;
     const bool slab = H.stencil_mode == kModeFused && is_slab_variant(H.fused_variant);
-    a.coef_kind = (H.stencil_mode == kModeStream || H.stencil_mode == kModeVec || slab) ? H.coef_kind : kCoefNative;
+    const bool compact = H.stencil_mode == kModeStream || H.stencil_mode == kModeVec || slab ||
+                         (H.stencil_mode == kModeSimple && H.auto_form);
+    a.coef_kind = compact ? H.coef_kind : kCoefNative;
+    a.unit_alpha = H.unit_alpha;
+    for (int q = 0; q < 2; ++q) a.a0[q] = H.a0[q];
     for (int q = 0; q < 4; ++q) a.cq[q] = H.cq[q].as<unsigned short>();
     for (int q = 0; q < 16; ++q) a.cs[q] = H.cs[q];
     return a;
@@ -694,6 +737,33 @@ void compact_coeffs(Handle& H) {
     }
     ck(cudaGetLastError(), "compact coefficients");
     ck(cudaStreamSynchronize(H.stream), "compact coefficients sync");
+}
+
+// Whether alpha follows from beta on both sides (lossless coefficients), in
+// the storage the kernels read: 1 wherever beta != 0, one value a0 elsewhere
+// (0: PEC edges frozen at zero; 1: entries that keep their value).  Padding
+// entries have alpha = beta = 0 and hold +0, which 0 x 0 and 1 x 0 both keep.
+void find_unit_alpha(Handle& H) {
+    H.unit_alpha = 0;
+    if (!H.coeffs_set) return;
+    if (!H.scan.p) H.scan.alloc(2 * sizeof(int), false);
+    ck(cudaMemsetAsync(H.scan.p, 0, H.scan.bytes, H.stream), "coefficient scan");
+    const auto scan = [&](auto args) {
+        args.coef_kind = H.coef_kind;
+        launch_unit_alpha(args, H.scan.as<int>(), H.stream);
+    };
+    if (H.prec == 4)
+        scan(stencil_args<float>(H));
+    else
+        scan(stencil_args<double>(H));
+    H.launches++;
+    ck(cudaGetLastError(), "coefficient scan");
+    int f[2];
+    ck(cudaMemcpyAsync(f, H.scan.p, sizeof(f), cudaMemcpyDeviceToHost, H.stream), "coefficient scan D2H");
+    ck(cudaStreamSynchronize(H.stream), "coefficient scan sync");
+    if (f[0] == 3 || f[1] == 3) return;
+    for (int q = 0; q < 2; ++q) H.a0[q] = (f[q] & 1) ? 1.0f : 0.0f;
+    H.unit_alpha = 1;
 }
 
 PortsArgs ports_args(Handle& H) {
@@ -875,8 +945,11 @@ void plan_stencil(Handle& H) {
 // the bulk-copy pipeline on request, the batched kernel for B > 1.  A side
 // with dispersive materials takes its CPML corrections in separate passes
 // after the ADE update, so its stencil launch carries no faces.
+// In a step of the direct kernels, pa != null, the E launch steps the lumped
+// ports it can (H.lumped_in_E) and the H launch advances the step counter
+// when `advance` says so.
 template <typename T>
-void launch_half(Handle& H, int which) {
+void launch_half(Handle& H, int which, const PortsArgs* pa = nullptr, bool advance = false) {
     StencilArgs<T> sa = stencil_args<T>(H);
     if (H.disp[which].present() || (which == 1 && H.sibc.present())) sa.nfaces = 0;
     switch (H.stencil_mode) {
@@ -890,8 +963,18 @@ void launch_half(Handle& H, int which) {
             which == 0 ? launch_update_E_bulk<T>(sa, H.plan, H.status.as<int>(), H.stream)
                        : launch_update_H_bulk<T>(sa, H.plan, H.status.as<int>(), H.stream);
             break;
-        default:
-            which == 0 ? launch_update_E<T>(sa, H.stream) : launch_update_H<T>(sa, H.stream);
+        default: {
+            DirectArgs da{};
+            da.np = H.direct_np;
+            if (pa && which == 0 && H.lumped_in_E) {
+                da.n_lumped = (int)H.lumped.size();
+                for (int q = 0; q < da.n_lumped; ++q) da.lumped[q] = H.lumped_cell[q];
+                da.ports = H.d_lumped.as<LumpedDev>();
+                da.pa = *pa;
+            }
+            if (advance) da.advance = H.step.as<long long>();
+            launch_direct_half<T>(sa, da, which, H.stream);
+        }
     }
 }
 
@@ -1066,11 +1149,10 @@ int enqueue_step_fused(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_stage_all<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.d_dft.as<DftDev>(),
-                                (int)H.dft.size(), H.dft_stage_blocks, H.step.as<long long>(), H.stream);
-        launch_dft_flush_all(H.B, H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_flush_blocks, H.dft_flush_smem,
-                             H.step.as<long long>(), H.ticket.as<unsigned>(), H.stream);
-        n += 2;
+        launch_dft_step<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.d_dft.as<DftDev>(),
+                           (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), 0,
+                           H.ticket.as<unsigned>(), H.stream);
+        ++n;
     } else {
         launch_advance(H.step.as<long long>(), H.stream);
         ++n;
@@ -1095,7 +1177,7 @@ int enqueue_step(Handle& H) {
         launch_sibc_save<T>(H.Hc().as<T>(), H.e_block(), H.B, H.sibc.dev, H.stream);
         ++n;
     }
-    launch_half<T>(H, 0);
+    launch_half<T>(H, 0, &pa);
     ++n;
     n += disp_complete<T>(H, 0);
     for (auto& pw : H.pws) {
@@ -1113,11 +1195,15 @@ int enqueue_step(Handle& H) {
                        (int)((H.cap + kConvChunk - 1) / kConvChunk), H.stream);
         n += 2;
     }
-    if (!H.lumped.empty()) {
+    const bool direct = H.stencil_mode == kModeSimple;
+    if (!H.lumped.empty() && !(direct && H.lumped_in_E)) {
         launch_lumped<T>(H.Ec().as<T>(), pa, H.d_lumped.as<LumpedDev>(), (int)H.lumped.size(), H.stream);
         ++n;
     }
-    launch_half<T>(H, 1);
+    // after this only the plane waves read the counter, and the monitors,
+    // which are told
+    const bool advance = direct && H.pws.empty();
+    launch_half<T>(H, 1, &pa, advance);
     ++n;
     n += disp_complete<T>(H, 1);
     for (auto& pw : H.pws) {
@@ -1125,14 +1211,11 @@ int enqueue_step(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        // stage + flush of all monitors; the flush launch advances the step
-        launch_dft_stage_all<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B,
-                                H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_stage_blocks, H.step.as<long long>(),
-                                H.stream);
-        launch_dft_flush_all(H.B, H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_flush_blocks, H.dft_flush_smem,
-                             H.step.as<long long>(), H.ticket.as<unsigned>(), H.stream);
-        n += 2;
-    } else {
+        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.d_dft.as<DftDev>(),
+                           (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), advance ? 1 : 0,
+                           H.ticket.as<unsigned>(), H.stream);
+        ++n;
+    } else if (!advance) {
         launch_advance(H.step.as<long long>(), H.stream);
         ++n;
     }
@@ -1273,6 +1356,95 @@ void run_steps(Handle& H, long long nsteps) {
     }
     H.launches += (long long)per * nsteps;
     H.steps_done += nsteps;
+}
+
+// Switches the stencil form between steps.
+void set_form(Handle& H, int kind, int variant, int ichunk) {
+    if (kind < kModeSimple || kind > kModeFused) fail(FITB_ERR_ARG, "stencil kind %d", kind);
+    if (ichunk < 0) fail(FITB_ERR_ARG, "ichunk %d", ichunk);
+    const bool compact = H.coef_kind != kCoefNative;
+    if (compact && kind != kModeStream && kind != kModeVec &&
+        !(kind == kModeFused && is_slab_variant(variant) && H.coef_kind == kCoefF16 && H.prec == 4))
+        fail(FITB_ERR_STATE,
+             "compact coefficient storage needs the stream or vec stencil kernels (float16: also the float32 slab "
+             "step)");
+    if ((kind == kModeStream || kind == kModeVec) && !stream_batch_supported(H.B))
+        fail(FITB_ERR_ARG, "the stream / vec kernels take 1, 2, 4, 8 or 16 field sets, not %d", H.B);
+    if (kind == kModeStream && !stream_variant_supported(H.B, variant))
+        fail(FITB_ERR_ARG, "stream stencil: variant %d / batch %d", variant, H.B);
+    if (kind == kModeVec && (H.B > 8 || variant < 0 || variant > 3))
+        fail(FITB_ERR_ARG, "vec stencil: variant %d / batch %d", variant, H.B);
+    if (kind == kModeFused) {
+        if (!fused_variant_ok(H.prec, variant)) fail(FITB_ERR_ARG, "fused variant %d", variant);
+        if (H.sibc.present()) fail(FITB_ERR_STATE, "SIBC walls need an in-place stencil mode");
+        if (!H.band.empty()) fail(FITB_ERR_STATE, "band DTBC ports need an in-place stencil mode");
+        if ((H.disp[0].present() || H.disp[1].present()) && !is_slab_variant(variant))
+            fail(FITB_ERR_STATE,
+                 "dispersive materials need an in-place stencil mode or the slab step (fused 16-25)");
+        if ((H.disp[0].present() || H.disp[1].present()) && !disp_clear_of_cpml(H))
+            fail(FITB_ERR_STATE, "the slab step takes dispersive materials only outside the CPML slabs");
+        if (is_tile_variant(variant) &&
+            !(H.prec == 4 ? tile_step_fits<float>(stencil_args<float>(H))
+                          : tile_step_fits<double>(stencil_args<double>(H))))
+            fail(FITB_ERR_ARG, "the tile step does not take this grid / CPML layout");
+        if (is_slab_variant(variant) && H.B % slab_nb_of(variant - kFusedSlabBase) != 0)
+            fail(FITB_ERR_ARG, "fused variant %d marches %d field sets per CTA: the batch of %d is not a multiple",
+                 variant, slab_nb_of(variant - kFusedSlabBase), H.B);
+        if (is_slab_variant(variant)) {
+            // any march depth the planner may pick: check the deepest and the shallowest
+            std::vector<int4> lists[kSlabLists];
+            const int np = H.g.nx + 1;
+            std::vector<int> depths;
+            for (int c = 12; c <= 20; ++c) depths.push_back(std::min(np, c));
+            if (ichunk > 0) depths.push_back(std::min(np, (int)ichunk));
+            for (int c : depths)
+                if (!slab_units_of(H, variant, c, lists))
+                    fail(FITB_ERR_ARG, "the slab step does not take this grid / CPML layout");
+        }
+    }
+    if (kind == kModeBulk && H.B != 1) fail(FITB_ERR_ARG, "the bulk-copy stencil takes one field set");
+    ck(cudaStreamSynchronize(H.stream), "configure sync");
+    int sms = 148;
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H.desc.device);
+    if (kind == kModeBulk) {
+        BulkPlan bp = H.prec == 4 ? plan_bulk<float>(H.g, sms) : plan_bulk<double>(H.g, sms);
+        if (bp.stages < 3) fail(FITB_ERR_ARG, "the bulk-copy stencil does not fit this grid's rows");
+        ck(H.prec == 4 ? prepare_bulk<float>(bp) : prepare_bulk<double>(bp), "bulk stencil smem attribute");
+        H.plan = bp;
+    }
+    const size_t blk = (size_t)H.e_block() * H.esz;
+    if (kind == kModeFused) {
+        ck(prepare_fused_any(H.prec, variant), "fused step smem attribute");
+        if (!H.e2.p) H.e2.alloc(blk * H.B);
+        if (!H.h2.p) H.h2.alloc(blk * H.B);
+        for (auto& f : H.faces)
+            if (!f->psi2.p) {
+                f->psi2.alloc(f->psi.bytes);
+                f->dev.psi_next = f->psi2.p;
+            }
+        H.fused_variant = variant;
+    } else if (H.stencil_mode == kModeFused && H.cur == 1) {
+        // leave the fused step with the current fields in the first buffer set
+        ck(cudaMemcpyAsync(H.e.p, H.e2.p, blk * H.B, cudaMemcpyDeviceToDevice, H.stream), "fields copy");
+        ck(cudaMemcpyAsync(H.h.p, H.h2.p, blk * H.B, cudaMemcpyDeviceToDevice, H.stream), "fields copy");
+        for (auto& f : H.faces)
+            ck(cudaMemcpyAsync(f->psi.p, f->psi2.p, f->psi.bytes, cudaMemcpyDeviceToDevice, H.stream), "psi copy");
+        ck(cudaStreamSynchronize(H.stream), "configure copy sync");
+        H.cur = 0;
+    }
+    if (kind == kModeVec) H.vec_variant = variant;
+    if (kind == kModeStream) H.stream_variant = compact ? 0 : variant;
+    H.stencil_mode = kind;
+    H.direct_np = ichunk;
+    plan_stencil(H);
+    if (ichunk > 0) {
+        const int nplanes = H.g.nx + 1;
+        const int c = std::min(ichunk, nplanes);
+        H.splan.ichunk = c;
+        H.splan.grid_z = (nplanes + c - 1) / c;
+    }
+    H.port_tables_dirty = true;
+    invalidate_graphs(H);
 }
 
 template <typename T>
@@ -1634,13 +1806,16 @@ int fitb_create(const fitb_desc* desc, fitb_handle** out) {
     H.status.alloc(sizeof(int));
     H.ticket.alloc(sizeof(unsigned));
     {
-        // FITB_STENCIL selects the stencil kernels: "stream" (default),
+        // FITB_STENCIL selects the stencil kernels: unset, the engine's own
+        // choice (the direct kernels); "simple" (the same kernels, chosen),
         // "fused" (E and H in one pass over ping-pong buffers;
         // FITB_FUSED_VARIANT picks the kernel form), "vec" (vectorised planes;
         // FITB_VEC_VARIANT picks the vector width and register cap), "bulk"
-        // (cp.async.bulk pipeline, one field set) or "simple".
+        // (cp.async.bulk pipeline, one field set), else the stream kernels
+        // where they take the batch.
         const char* mode = getenv("FITB_STENCIL");
-        const std::string m = mode ? mode : "stream";
+        const std::string m = mode ? mode : "simple";
+        H.auto_form = mode == nullptr;
         H.stencil_mode = fitb::kModeSimple;
         if (H.B == 1 && m == "bulk") {
             int sms = 148;
@@ -1718,6 +1893,7 @@ int fitb_set_coeffs(fitb_handle* h, const double* alpha_e, const double* beta_e,
     fitb::comp_max(H, beta_h, 3, H.coef_max[3]);
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
+    fitb::find_unit_alpha(H);
     H.port_tables_dirty = true;  // the slab step's dead-unit plan reads the coefficients
     fitb::invalidate_graphs(H);
     FITB_CATCH
@@ -1772,6 +1948,7 @@ int fitb_build_materials(fitb_handle* h, const double* dx, const double* dy, con
     H.launches += 5;
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
+    fitb::find_unit_alpha(H);
     H.port_tables_dirty = true;
     fitb::invalidate_graphs(H);
     FITB_CATCH
@@ -1826,6 +2003,7 @@ int fitb_set_coeffs_native(fitb_handle* h, const void* alpha_e, const void* beta
     }
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
+    fitb::find_unit_alpha(H);
     H.port_tables_dirty = true;  // the slab step's dead-unit plan reads the coefficients
     fitb::invalidate_graphs(H);
     FITB_CATCH
@@ -1836,8 +2014,9 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind) {
     Handle& H = H_of(h);
     if (kind < fitb::kCoefNative || kind > fitb::kCoefBF16) fail(FITB_ERR_ARG, "coefficient storage kind %d", kind);
     const bool slab = H.stencil_mode == fitb::kModeFused && fitb::is_slab_variant(H.fused_variant);
-    if (kind != fitb::kCoefNative && H.stencil_mode != fitb::kModeStream && H.stencil_mode != fitb::kModeVec &&
-        !(slab && kind == fitb::kCoefF16 && H.prec == 4))
+    const bool own_choice = H.auto_form && fitb::stream_batch_supported(H.B);
+    if (kind != fitb::kCoefNative && !own_choice && H.stencil_mode != fitb::kModeStream &&
+        H.stencil_mode != fitb::kModeVec && !(slab && kind == fitb::kCoefF16 && H.prec == 4))
         fail(FITB_ERR_STATE,
              "compact coefficient storage needs the stream or vec stencil kernels (float16: also the float32 slab "
              "step)");
@@ -1847,6 +2026,7 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind) {
     }
     fitb::plan_stencil(H);
     fitb::compact_coeffs(H);
+    fitb::find_unit_alpha(H);
     fitb::invalidate_graphs(H);
     FITB_CATCH
 }
@@ -1854,91 +2034,8 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind) {
 int fitb_configure_stencil(fitb_handle* h, int32_t kind, int32_t variant, int32_t ichunk) {
     FITB_TRY
     Handle& H = H_of(h);
-    if (kind < fitb::kModeSimple || kind > fitb::kModeFused) fail(FITB_ERR_ARG, "stencil kind %d", kind);
-    if (ichunk < 0) fail(FITB_ERR_ARG, "ichunk %d", ichunk);
-    const bool compact = H.coef_kind != fitb::kCoefNative;
-    if (compact && kind != fitb::kModeStream && kind != fitb::kModeVec &&
-        !(kind == fitb::kModeFused && fitb::is_slab_variant(variant) && H.coef_kind == fitb::kCoefF16 && H.prec == 4))
-        fail(FITB_ERR_STATE,
-             "compact coefficient storage needs the stream or vec stencil kernels (float16: also the float32 slab "
-             "step)");
-    if ((kind == fitb::kModeStream || kind == fitb::kModeVec) && !fitb::stream_batch_supported(H.B))
-        fail(FITB_ERR_ARG, "the stream / vec kernels take 1, 2, 4, 8 or 16 field sets, not %d", H.B);
-    if (kind == fitb::kModeStream && !fitb::stream_variant_supported(H.B, variant))
-        fail(FITB_ERR_ARG, "stream stencil: variant %d / batch %d", variant, H.B);
-    if (kind == fitb::kModeVec && (H.B > 8 || variant < 0 || variant > 3))
-        fail(FITB_ERR_ARG, "vec stencil: variant %d / batch %d", variant, H.B);
-    if (kind == fitb::kModeFused) {
-        if (!fitb::fused_variant_ok(H.prec, variant)) fail(FITB_ERR_ARG, "fused variant %d", variant);
-        if (H.sibc.present()) fail(FITB_ERR_STATE, "SIBC walls need an in-place stencil mode");
-        if (!H.band.empty()) fail(FITB_ERR_STATE, "band DTBC ports need an in-place stencil mode");
-        if ((H.disp[0].present() || H.disp[1].present()) && !fitb::is_slab_variant(variant))
-            fail(FITB_ERR_STATE,
-                 "dispersive materials need an in-place stencil mode or the slab step (fused 16-25)");
-        if ((H.disp[0].present() || H.disp[1].present()) && !fitb::disp_clear_of_cpml(H))
-            fail(FITB_ERR_STATE, "the slab step takes dispersive materials only outside the CPML slabs");
-        if (fitb::is_tile_variant(variant) &&
-            !(H.prec == 4 ? fitb::tile_step_fits<float>(fitb::stencil_args<float>(H))
-                          : fitb::tile_step_fits<double>(fitb::stencil_args<double>(H))))
-            fail(FITB_ERR_ARG, "the tile step does not take this grid / CPML layout");
-        if (fitb::is_slab_variant(variant) && H.B % fitb::slab_nb_of(variant - fitb::kFusedSlabBase) != 0)
-            fail(FITB_ERR_ARG, "fused variant %d marches %d field sets per CTA: the batch of %d is not a multiple",
-                 variant, fitb::slab_nb_of(variant - fitb::kFusedSlabBase), H.B);
-        if (fitb::is_slab_variant(variant)) {
-            // any march depth the planner may pick: check the deepest and the shallowest
-            std::vector<int4> lists[fitb::kSlabLists];
-            const int np = H.g.nx + 1;
-            std::vector<int> depths;
-            for (int c = 12; c <= 20; ++c) depths.push_back(std::min(np, c));
-            if (ichunk > 0) depths.push_back(std::min(np, (int)ichunk));
-            for (int c : depths)
-                if (!fitb::slab_units_of(H, variant, c, lists))
-                    fail(FITB_ERR_ARG, "the slab step does not take this grid / CPML layout");
-        }
-    }
-    if (kind == fitb::kModeBulk && H.B != 1) fail(FITB_ERR_ARG, "the bulk-copy stencil takes one field set");
-    ck(cudaStreamSynchronize(H.stream), "configure sync");
-    int sms = 148;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, H.desc.device);
-    if (kind == fitb::kModeBulk) {
-        fitb::BulkPlan bp = H.prec == 4 ? fitb::plan_bulk<float>(H.g, sms) : fitb::plan_bulk<double>(H.g, sms);
-        if (bp.stages < 3) fail(FITB_ERR_ARG, "the bulk-copy stencil does not fit this grid's rows");
-        ck(H.prec == 4 ? fitb::prepare_bulk<float>(bp) : fitb::prepare_bulk<double>(bp), "bulk stencil smem attribute");
-        H.plan = bp;
-    }
-    const size_t blk = (size_t)H.e_block() * H.esz;
-    if (kind == fitb::kModeFused) {
-        ck(fitb::prepare_fused_any(H.prec, variant), "fused step smem attribute");
-        if (!H.e2.p) H.e2.alloc(blk * H.B);
-        if (!H.h2.p) H.h2.alloc(blk * H.B);
-        for (auto& f : H.faces)
-            if (!f->psi2.p) {
-                f->psi2.alloc(f->psi.bytes);
-                f->dev.psi_next = f->psi2.p;
-            }
-        H.fused_variant = variant;
-    } else if (H.stencil_mode == fitb::kModeFused && H.cur == 1) {
-        // leave the fused step with the current fields in the first buffer set
-        ck(cudaMemcpyAsync(H.e.p, H.e2.p, blk * H.B, cudaMemcpyDeviceToDevice, H.stream), "fields copy");
-        ck(cudaMemcpyAsync(H.h.p, H.h2.p, blk * H.B, cudaMemcpyDeviceToDevice, H.stream), "fields copy");
-        for (auto& f : H.faces)
-            ck(cudaMemcpyAsync(f->psi.p, f->psi2.p, f->psi.bytes, cudaMemcpyDeviceToDevice, H.stream), "psi copy");
-        ck(cudaStreamSynchronize(H.stream), "configure copy sync");
-        H.cur = 0;
-    }
-    if (kind == fitb::kModeVec) H.vec_variant = variant;
-    if (kind == fitb::kModeStream) H.stream_variant = compact ? 0 : variant;
-    H.stencil_mode = kind;
-    fitb::plan_stencil(H);
-    if (ichunk > 0) {
-        const int nplanes = H.g.nx + 1;
-        const int c = std::min(ichunk, nplanes);
-        H.ichunk = c;
-        H.splan.ichunk = c;
-        H.splan.grid_z = (nplanes + c - 1) / c;
-    }
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::set_form(H, kind, variant, ichunk);
+    H.auto_form = false;
     FITB_CATCH
 }
 
@@ -1983,7 +2080,7 @@ int fitb_get_stencil(fitb_handle* h, int32_t* out) {
              : H.stencil_mode == fitb::kModeFused ? H.fused_variant
              : H.stencil_mode == fitb::kModeStream ? H.stream_variant
                                                    : 0;
-    out[2] = planned ? H.splan.ichunk : (H.stencil_mode == fitb::kModeBulk ? H.plan.ichunk : H.ichunk);
+    out[2] = planned ? H.splan.ichunk : (H.stencil_mode == fitb::kModeBulk ? H.plan.ichunk : std::max(1, H.direct_np));
     out[3] = planned ? H.splan.grid_x : 0;
     out[4] = planned ? H.splan.grid_y : 0;
     out[5] = planned ? H.splan.grid_z : 0;
@@ -2160,6 +2257,7 @@ int fitb_add_modal_port(fitb_handle* h, const fitb_modal_desc* d, int32_t* out_i
     fitb::upload(mp->port_e, pe);
     mp->port_e_host = pe;
     fitb::upload(mp->int_e, ie);
+    mp->int_e_host = ie;
     fitb::upload(mp->port_h, ph);
     fitb::upload(mp->me_port, std::vector<double>(d->me_port, d->me_port + ne));
     fitb::upload(mp->me_int, std::vector<double>(d->me_int, d->me_int + ne));

@@ -61,6 +61,7 @@ struct FaceDev {
     void* psi;      // [B][4][slab] field dtype: E1, E2, H1, H2
     void* psi_next; // fused step: the buffer the new psi goes to
     const unsigned char* air;  // [4][slab] 0/1
+    int masked;     // some air entry is 0 (PEC inside the slab)
     const void* bcc;           // [3][n] field dtype: b, c, ck
 };
 
@@ -87,6 +88,10 @@ struct StencilArgs {
     int coef_kind;
     const unsigned short* cq[4];
     float cs[16];
+    // Lossless coefficients: alpha is 1 wherever beta != 0 and a0[side]
+    // elsewhere (E, H), so the kernels that know this do not read it.
+    int unit_alpha;
+    float a0[2];
 };
 
 constexpr int kCoefNative = 0, kCoefF16 = 1, kCoefBF16 = 2;
@@ -94,11 +99,6 @@ constexpr int kCoefNative = 0, kCoefF16 = 1, kCoefBF16 = 2;
 // dst[q] = 16-bit(src[q] * inv_scale), round to nearest even.
 template <typename T>
 void launch_compact(const T* src, unsigned short* dst, long long n, float inv_scale, int coef_kind, cudaStream_t s);
-
-template <typename T>
-void launch_update_E(const StencilArgs<T>& a, cudaStream_t s);
-template <typename T>
-void launch_update_H(const StencilArgs<T>& a, cudaStream_t s);
 
 // Software-pipelined register stencil, batched over B in {1, 2, 4, 8, 16}
 // field sets (the default kernels).
@@ -483,18 +483,18 @@ struct DftDev {
     float2* bins;         // [B][ncomp][nf][ncell]
     float2* cmp;          // Kahan compensation, same shape
     double dt;
-    int sblk0, sblk;      // this monitor's blocks in the merged stage launch
-    int fblk0, fblk;      // and in the merged flush launch
+    int sblk0, sblk;      // this monitor's blocks in the merged launch
 };
 
 int dft_blocks(long long work);
-// One launch stages every monitor; one launch flushes every full monitor and
-// advances the step counter (its last CTA, through `ticket`).
+// One launch per step stages every monitor's samples and flushes the full
+// ones (dynamic shared memory for the largest monitor's phasors).  done = 1:
+// the step counter is already advanced; 0: this launch advances it (its last
+// CTA, through `ticket`).
 template <typename T>
-void launch_dft_stage_all(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                          const DftDev* devs, int nmon, int nblocks, const long long* step, cudaStream_t s);
-void launch_dft_flush_all(int B, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step,
-                          unsigned* ticket, cudaStream_t s);
+void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
+                     const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
+                     unsigned* ticket, cudaStream_t s);
 // Host-requested flush of the first kc slots of one monitor.
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s);
 

@@ -8,12 +8,11 @@
 //
 // Here each recorded step only stages the interpolated float32 samples and
 // the float64-evaluated phasors exp(j w t) dt_w of that step into a block of
-// K slots (k_dft_stage_all).  When a monitor's block is full,
-// k_dft_flush_all forms sum_s w_s[f] x_s for every bin in registers and adds
-// it once to the bins (optionally Kahan-compensated): the complex bins are
-// read and written once per K recorded steps instead of once per step.
-// All monitors share one stage launch and one flush launch per step; the
-// last CTA of the flush launch advances the device step counter.
+// K slots.  On the step that fills the block, the thread that staged a cell's
+// samples forms sum_s w_s[f] x_s for every bin of that cell in registers and
+// adds it once to the bins (optionally Kahan-compensated): the complex bins
+// are read and written once per K recorded steps instead of once per step.
+// All monitors share this one launch per step (k_dft_step).
 #include "fitb_common.cuh"
 
 namespace fitb {
@@ -70,110 +69,109 @@ __device__ __forceinline__ double interp_sample(const T* E, const T* H, long lon
     }
 }
 
-__device__ __forceinline__ int monitor_of_block(const DftDev* devs, int nmon, bool stage) {
+__device__ __forceinline__ int monitor_of_block(const DftDev* devs, int nmon) {
     int m = 0;
-    while (m + 1 < nmon && (int)blockIdx.x >= (stage ? devs[m + 1].sblk0 : devs[m + 1].fblk0)) ++m;
+    while (m + 1 < nmon && (int)blockIdx.x >= devs[m + 1].sblk0) ++m;
     return m;
 }
 
+// Adds kc staged samples x[s * xs] (s < n_st) and, at s = kc - 1, `last` to
+// the bins of one cell-component: bins bi + f * ncell, phasors sw.
+__device__ __forceinline__ void flush_cell(const DftDev& d, int kc, int tsel, const float* x, long long xs, int n_st,
+                                           float last, long long bi, const float2* sw) {
+    float v[kMaxK];
+#pragma unroll
+    for (int s = 0; s < kMaxK; ++s) v[s] = s < n_st ? x[s * xs] : (s == kc - 1 ? last : 0.0f);
+    for (int f = 0; f < d.nf; ++f, bi += d.ncell) {
+        float re = 0.0f, im = 0.0f;
+#pragma unroll
+        for (int s = 0; s < kMaxK; ++s) {
+            if (s < kc) {
+                const float2 w = sw[(s * 2 + tsel) * d.nf + f];
+                re = fmaf(w.x, v[s], re);
+                im = fmaf(w.y, v[s], im);
+            }
+        }
+        float2 acc = d.bins[bi];
+        if (d.kahan) {
+            float2 cm = d.cmp[bi];
+            const float yr = re - cm.x, yi = im - cm.y;
+            const float tr = acc.x + yr, ti = acc.y + yi;
+            cm.x = (tr - acc.x) - yr;
+            cm.y = (ti - acc.y) - yi;
+            acc.x = tr;
+            acc.y = ti;
+            d.cmp[bi] = cm;
+        } else {
+            acc.x += re;
+            acc.y += im;
+        }
+        d.bins[bi] = acc;
+    }
+}
+
+// One step of every monitor.  The step counter is *step - done: done = 1 when
+// an earlier kernel of the step has advanced it; otherwise the last CTA of
+// this launch does, through `ticket`.  Staging and flushing were two launches
+// before, the second one empty on K - 1 of K steps: on a 97 x 104 x 89 mesh
+// with three planes of 16 frequencies the two cost 13 us per step.
 template <typename T>
-__global__ void __launch_bounds__(kThreads)
-    k_dft_stage_all(const T* __restrict__ e, const T* __restrict__ h, long long e_block, long long h_block, Geom g,
-                    int B, const DftDev* __restrict__ devs, int nmon, const long long* __restrict__ step) {
-    const DftDev& d = devs[monitor_of_block(devs, nmon, true)];
-    const int lb = blockIdx.x - d.sblk0;
-    const long long n = *step;
-    if (n % d.stride) return;
-    const long long cnt = recorded_upto(n, d.stride) - recorded_upto(*d.base - 1, d.stride);
-    const int slot = (int)((cnt - 1) % d.K);
-    if (lb == 0) {
-        const double tE = (double)n * d.dt;
-        const double tH = tE + 0.5 * d.dt;
-        const double dtw = (double)d.stride * d.dt;
-        for (int q = threadIdx.x; q < 2 * d.nf; q += blockDim.x) {
-            const int f = q % d.nf;
-            const double t = (q < d.nf) ? tE : tH;
-            double sn, cs;
-            sincos(d.omega[f] * t, &sn, &cs);
-            d.wst[((long long)slot * 2 + (q / d.nf)) * d.nf + f] = make_float2((float)(cs * dtw), (float)(sn * dtw));
-        }
-    }
-    const long long total = (long long)d.ncomp * d.ncell;
-    for (long long t = lb * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)d.sblk * blockDim.x) {
-        const int ci = (int)(t / d.ncell);
-        const long long cell = t % d.ncell;
-        const int kk = (int)(cell % d.nk);
-        const long long r = cell / d.nk;
-        const int jj = (int)(r % d.nj);
-        const int ii = (int)(r / d.nj);
-        const int c = d.comps[ci];
-        for (int b = 0; b < B; ++b) {
-            const double v = interp_sample<T>(e + (long long)b * e_block, h + (long long)b * h_block, g.vol, g, d, c,
-                                              d.i0 + ii, d.j0 + jj, d.k0 + kk);
-            d.stage[(((long long)b * d.K + slot) * d.ncomp + ci) * d.ncell + cell] = (float)v;
-        }
-    }
-}
-
-// Adds the kc staged slots of one monitor to its bins (threads of the
-// monitor's blocks, lb = local block index, nb = the monitor's block count).
-__device__ void flush_slots(int B, const DftDev& d, int kc, int lb, int nb, float2* sw) {
-    for (int q = threadIdx.x; q < kc * 2 * d.nf; q += blockDim.x) sw[q] = d.wst[q];
-    __syncthreads();
-    const long long per_b = (long long)d.ncomp * d.ncell;
-    const long long total = (long long)B * per_b;
-    for (long long t = lb * (long long)blockDim.x + threadIdx.x; t < total; t += (long long)nb * blockDim.x) {
-        const int b = (int)(t / per_b);
-        const long long r = t % per_b;
-        const int ci = (int)(r / d.ncell);
-        const long long cell = r % d.ncell;
-        const int tsel = (d.comps[ci] < 3) ? 0 : 1;
-        float x[kMaxK];
-#pragma unroll
-        for (int s = 0; s < kMaxK; ++s)
-            x[s] = (s < kc) ? d.stage[(((long long)b * d.K + s) * d.ncomp + ci) * d.ncell + cell] : 0.0f;
-        for (int f = 0; f < d.nf; ++f) {
-            float re = 0.0f, im = 0.0f;
-#pragma unroll
-            for (int s = 0; s < kMaxK; ++s) {
-                if (s < kc) {
-                    const float2 w = sw[(s * 2 + tsel) * d.nf + f];
-                    re = fmaf(w.x, x[s], re);
-                    im = fmaf(w.y, x[s], im);
-                }
-            }
-            const long long bi = (((long long)b * d.ncomp + ci) * d.nf + f) * d.ncell + cell;
-            float2 acc = d.bins[bi];
-            if (d.kahan) {
-                float2 cm = d.cmp[bi];
-                const float yr = re - cm.x, yi = im - cm.y;
-                const float tr = acc.x + yr, ti = acc.y + yi;
-                cm.x = (tr - acc.x) - yr;
-                cm.y = (ti - acc.y) - yi;
-                acc.x = tr;
-                acc.y = ti;
-                d.cmp[bi] = cm;
-            } else {
-                acc.x += re;
-                acc.y += im;
-            }
-            d.bins[bi] = acc;
-        }
-    }
-}
-
-__global__ void __launch_bounds__(kThreads)
-    k_dft_flush_all(int B, const DftDev* __restrict__ devs, int nmon, long long* step, unsigned* ticket) {
+__global__ void __launch_bounds__(kThreads, 3)
+    k_dft_step(const T* __restrict__ e, const T* __restrict__ h, long long e_block, long long h_block, Geom g, int B,
+               const DftDev* __restrict__ devs, int nmon, long long* step, int done, unsigned* ticket) {
     extern __shared__ float2 sw[];
-    const DftDev& d = devs[monitor_of_block(devs, nmon, false)];
-    const int lb = blockIdx.x - d.fblk0;
-    const long long n = *step;
-    bool go = (n % d.stride) == 0;
-    if (go) {
+    const DftDev& d = devs[monitor_of_block(devs, nmon)];
+    const int lb = blockIdx.x - d.sblk0;
+    const long long n = *step - done;
+    if (n % d.stride == 0) {
         const long long cnt = recorded_upto(n, d.stride) - recorded_upto(*d.base - 1, d.stride);
-        go = (int)((cnt - 1) % d.K) == d.K - 1;
+        const int slot = (int)((cnt - 1) % d.K);
+        const bool flush = slot == d.K - 1;
+        // this step's phasors: for the later steps of the block, and (every
+        // CTA for itself) for the flush
+        if (lb == 0 || flush) {
+            const double tE = (double)n * d.dt;
+            const double tH = tE + 0.5 * d.dt;
+            const double dtw = (double)d.stride * d.dt;
+            for (int q = threadIdx.x; q < 2 * d.nf; q += blockDim.x) {
+                const int f = q % d.nf;
+                const double t = (q < d.nf) ? tE : tH;
+                double sn, cs;
+                sincos(d.omega[f] * t, &sn, &cs);
+                const float2 w = make_float2((float)(cs * dtw), (float)(sn * dtw));
+                const long long at = ((long long)slot * 2 + (q / d.nf)) * d.nf + f;
+                if (flush)
+                    sw[at] = w;
+                else
+                    d.wst[at] = w;
+            }
+        }
+        if (flush) {
+            for (int q = threadIdx.x; q < (d.K - 1) * 2 * d.nf; q += blockDim.x) sw[q] = d.wst[q];
+            __syncthreads();
+        }
+        const int total = d.ncomp * (int)d.ncell;
+        for (int t = lb * kThreads + threadIdx.x; t < total; t += d.sblk * kThreads) {
+            const int ci = t / (int)d.ncell;
+            const int cell = t - ci * (int)d.ncell;
+            const int kk = cell % d.nk;
+            const int r = cell / d.nk;
+            const int jj = r % d.nj;
+            const int ii = r / d.nj;
+            const int c = d.comps[ci];
+            for (int b = 0; b < B; ++b) {
+                const float v = (float)interp_sample<T>(e + (long long)b * e_block, h + (long long)b * h_block, g.vol,
+                                                        g, d, c, d.i0 + ii, d.j0 + jj, d.k0 + kk);
+                float* x = d.stage + ((long long)b * d.K * d.ncomp + ci) * d.ncell + cell;
+                if (flush)
+                    flush_cell(d, d.K, c < 3 ? 0 : 1, x, (long long)total, d.K - 1, v,
+                               ((long long)(b * d.ncomp + ci) * d.nf) * d.ncell + cell, sw);
+                else
+                    x[(long long)slot * total] = v;
+            }
+        }
     }
-    if (go) flush_slots(B, d, d.K, lb, d.fblk, sw);
+    if (done) return;
     // The last CTA to finish advances the step counter: every CTA has read
     // it above, and the next launch in the stream starts after this one.
     __syncthreads();
@@ -187,9 +185,21 @@ __global__ void __launch_bounds__(kThreads)
     }
 }
 
+// The first kc slots of one monitor, on request.
 __global__ void __launch_bounds__(kThreads) k_dft_flush_forced(int B, DftDev d, int kc) {
     extern __shared__ float2 sw[];
-    flush_slots(B, d, kc, blockIdx.x, gridDim.x, sw);
+    for (int q = threadIdx.x; q < kc * 2 * d.nf; q += blockDim.x) sw[q] = d.wst[q];
+    __syncthreads();
+    const long long per_b = (long long)d.ncomp * d.ncell;
+    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < B * per_b;
+         t += (long long)gridDim.x * blockDim.x) {
+        const int b = (int)(t / per_b);
+        const long long r = t % per_b;
+        const int ci = (int)(r / d.ncell);
+        const long long cell = r % d.ncell;
+        flush_cell(d, kc, d.comps[ci] < 3 ? 0 : 1, d.stage + ((long long)b * d.K * d.ncomp + ci) * d.ncell + cell,
+                   per_b, kc, 0.0f, ((long long)(b * d.ncomp + ci) * d.nf) * d.ncell + cell, sw);
+    }
 }
 
 }  // namespace
@@ -201,14 +211,10 @@ int dft_blocks(long long work) {
 }
 
 template <typename T>
-void launch_dft_stage_all(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                          const DftDev* devs, int nmon, int nblocks, const long long* step, cudaStream_t s) {
-    k_dft_stage_all<T><<<nblocks, kThreads, 0, s>>>(e, h, e_block, h_block, g, B, devs, nmon, step);
-}
-
-void launch_dft_flush_all(int B, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step,
-                          unsigned* ticket, cudaStream_t s) {
-    k_dft_flush_all<<<nblocks, kThreads, smem, s>>>(B, devs, nmon, step, ticket);
+void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
+                     const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
+                     unsigned* ticket, cudaStream_t s) {
+    k_dft_step<T><<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, devs, nmon, step, done, ticket);
 }
 
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s) {
@@ -216,9 +222,9 @@ void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s) {
     k_dft_flush_forced<<<dft_blocks((long long)B * d.ncomp * d.ncell), kThreads, smem, s>>>(B, d, kc);
 }
 
-template void launch_dft_stage_all<float>(const float*, const float*, long long, long long, const Geom&, int,
-                                          const DftDev*, int, int, const long long*, cudaStream_t);
-template void launch_dft_stage_all<double>(const double*, const double*, long long, long long, const Geom&, int,
-                                           const DftDev*, int, int, const long long*, cudaStream_t);
+template void launch_dft_step<float>(const float*, const float*, long long, long long, const Geom&, int,
+                                     const DftDev*, int, int, size_t, long long*, int, unsigned*, cudaStream_t);
+template void launch_dft_step<double>(const double*, const double*, long long, long long, const Geom&, int,
+                                      const DftDev*, int, int, size_t, long long*, int, unsigned*, cudaStream_t);
 
 }  // namespace fitb

@@ -12,6 +12,7 @@
 // All port arithmetic is float64, as in the reference; only the field
 // gathers/scatters touch the field dtype.
 #include "fitb_common.cuh"
+#include "lumped.cuh"
 
 namespace fitb {
 
@@ -60,32 +61,14 @@ __global__ void k_lumped(T* __restrict__ e, PortsArgs pa, const LumpedDev* __res
     T* E = e + (long long)b * pa.e_block;
     double v_total = 0.0;
     for (int q = 0; q < d.n_edges; ++q) v_total += d.sign[q] * (double)E[d.off[q]];
-    const double v_src = (n < d.n_src) ? d.src[(long long)b * d.n_src + n] : 0.0;
-    double* st = d.st + 4 * b;
-    const double dt = pa.dt_lumped;
-    const double i_prev = st[0];
-    double r_eq = (d.R >= 0.0) ? d.R : 0.0;
-    if (d.L >= 0.0) r_eq += 2.0 * d.L / dt;
-    if (d.C >= 0.0) r_eq += dt / (2.0 * d.C);
-    double v_hist = 0.0;
-    if (d.L >= 0.0) v_hist += -(2.0 * d.L / dt) * i_prev - st[1];
-    if (d.C >= 0.0) v_hist += st[2] + (dt / (2.0 * d.C)) * i_prev;
-    const double z_eff = r_eq + d.beta_sum;
-    const double i_port = (v_src - v_hist - v_total) / z_eff;
+    const double i_port = lumped_current(d, pa, b, n, v_total);
     for (int q = 0; q < d.n_edges; ++q) {
         const long long o = d.off[q];
         E[o] = (T)((double)E[o] + d.sign[q] * d.beta[q] * i_port);
     }
-    if (d.L >= 0.0) st[1] = (2.0 * d.L / dt) * (i_port - i_prev) - st[1];
-    if (d.C >= 0.0) st[2] = st[2] + (dt / (2.0 * d.C)) * (i_port + i_prev);
-    st[0] = i_port;
-    st[3] = i_port;
-    // Recorder: V re-projected from the corrected field, I = cached current.
     double v = 0.0;
     for (int q = 0; q < d.n_edges; ++q) v += d.sign[q] * (double)E[d.off[q]];
-    const long long r = ((long long)b * pa.rec.cap + n) * pa.rec.nch + d.channel;
-    pa.rec.V[r] = v * d.rec_scale;
-    pa.rec.I[r] = i_port * d.rec_scale;
+    lumped_record(d, pa, b, n, v, i_port);
 }
 
 // _interp_delayed (operator.py:1539-1562) on the source history

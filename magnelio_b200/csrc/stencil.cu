@@ -1,4 +1,5 @@
-// Leapfrog curl updates with the CFS-PML psi recursion fused in.
+// Leapfrog curl updates with the CFS-PML psi recursion fused in: the direct
+// form, one cell per thread.
 //
 //   E^{n+1} = aE * E^n + bE * (C^T h)      then, on CPML slabs,
 //             E += +-bE * (ck * dH + psi_E),  psi_E = air * (b psi_E + c dH)
@@ -10,180 +11,382 @@
 // CPMLBoundary.update_E / update_H (src/magnelio/boundaries/cpml.py:343-516).
 // The in-thread curl order is the reference's: curl = +H_a - H_a' - H_b + H_b'.
 //
-// Thread mapping: one thread per (j, k) column of the padded box, marching
-// over a chunk of i planes; k is the contiguous axis, so every warp issues
-// 128-byte coalesced row segments.  Each thread updates all three
-// components of its column for every field set b (coefficients are loaded
-// once per cell and reused across the batch).
-#include "fitb_common.cuh"
+// Thread mapping: a thread owns 16 bytes of consecutive k (4 float, 2 double
+// cells) of one field set; threads run along the flattened rows of one i plane
+// (the padded row pitch is a multiple of 8), blockIdx.y is the plane (np planes
+// per thread), threadIdx.y the field set: the sets of a cell share its
+// coefficients through the L1.  Nothing is staged and no thread waits for
+// another, so meshes whose state stays in the L2 (up to about 1.5 M cells in
+// float32: latency and instructions bound them, not HBM) keep the whole chip
+// busy where a march along i (the stream, tile and slab forms) leaves most of
+// it idle; large meshes stream at the HBM rate (256^3 without CPML, float32:
+// 256 us per step, 96 B per cell at 0.98 of the measured copy rate).  Cells
+// per second, direct / stream / slab step: 36.8 / 14.4 / 15.0 G at 0.9 M cells,
+// 52 / 28 / 39 G at 10.9 M, 57.7 / 41.0 / 46.7 G at 105 M (CPML all round);
+// four field sets of 8 M cells 55 / 40 / 42 G.
+#include "direct.cuh"
+#include "lumped.cuh"
+
+#include <cuda_bf16.h>
+#include <cuda_fp16.h>
+
+#include <algorithm>
+#include <type_traits>
 
 namespace fitb {
 
 namespace {
 
-constexpr int kBX = 32;
-constexpr int kBY = 8;
+constexpr int kDirectThreads = 128;
 
-template <typename T>
-__device__ __forceinline__ long long slab_index(const FaceDev& f, int l, int i, int j, int k) {
-    const int a = (f.axis == 0) ? l : i;
-    const int b = (f.axis == 1) ? l : j;
-    const int c = (f.axis == 2) ? l : k;
-    return ((long long)a * f.dJ + b) * f.pk + c;
+// V consecutive cells of one array.
+template <typename T, int V>
+struct Vec {
+    T v[V];
+};
+
+template <int V>
+__device__ __forceinline__ Vec<float, V> ldv(const float* p) {
+    static_assert(V == 1 || V == 4, "16 bytes or one cell");
+    if constexpr (V == 1) return {{*p}};
+    if constexpr (V == 4) {
+        const float4 q = *reinterpret_cast<const float4*>(p);
+        return {{q.x, q.y, q.z, q.w}};
+    }
+}
+template <int V>
+__device__ __forceinline__ Vec<double, V> ldv(const double* p) {
+    static_assert(V == 1 || V == 2, "16 bytes or one cell");
+    if constexpr (V == 1) return {{*p}};
+    if constexpr (V == 2) {
+        const double2 q = *reinterpret_cast<const double2*>(p);
+        return {{q.x, q.y}};
+    }
+}
+template <int V>
+__device__ __forceinline__ void stv(float* p, const Vec<float, V>& a) {
+    if constexpr (V == 1) *p = a.v[0];
+    if constexpr (V == 4) *reinterpret_cast<float4*>(p) = make_float4(a.v[0], a.v[1], a.v[2], a.v[3]);
+}
+template <int V>
+__device__ __forceinline__ void stv(double* p, const Vec<double, V>& a) {
+    if constexpr (V == 1) *p = a.v[0];
+    if constexpr (V == 2) *reinterpret_cast<double2*>(p) = make_double2(a.v[0], a.v[1]);
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBX* kBY) k_update_E(const StencilArgs<T> p) {
+template <typename T, int CK>
+__device__ __forceinline__ T decode16(unsigned short u, float scale) {
+    if constexpr (CK == kCoefF16) return (T)__half2float(__ushort_as_half(u)) * (T)scale;
+    return (T)__bfloat162float(__ushort_as_bfloat16(u)) * (T)scale;
+}
+
+// Entry o of one stored coefficient array.
+template <typename T, int CK>
+__device__ __forceinline__ T coef_at(const T* __restrict__ a, const unsigned short* __restrict__ q, float scale,
+                                     long long o) {
+    if constexpr (CK == kCoefNative) return __ldg(a + o);
+    return decode16<T, CK>(__ldg(q + o), scale);
+}
+
+template <typename T, int V, int CK>
+__device__ __forceinline__ Vec<T, V> coef_vec(const T* a, const unsigned short* q, float scale, long long o) {
+    if constexpr (CK == kCoefNative) {
+        return ldv<V>(a + o);
+    } else {
+        Vec<T, V> r;
+        unsigned short u[V];
+        if constexpr (V == 4) {
+            const ushort4 w = *reinterpret_cast<const ushort4*>(q + o);
+            u[0] = w.x, u[1] = w.y, u[2] = w.z, u[3] = w.w;
+        } else if constexpr (V == 2) {
+            const ushort2 w = *reinterpret_cast<const ushort2*>(q + o);
+            u[0] = w.x, u[1] = w.y;
+        } else {
+            u[0] = q[o];
+        }
+#pragma unroll
+        for (int c = 0; c < V; ++c) r.v[c] = decode16<T, CK>(u[c], scale);
+        return r;
+    }
+}
+
+// The update coefficients of a thread's cells and side (0: E, 1: H).  UA:
+// alpha is one wherever beta is not zero and a0 elsewhere, so it is not read.
+template <typename T, int V, int CK, bool UA>
+__device__ __forceinline__ void load_cell_coef(const StencilArgs<T>& p, int side, int o, Vec<T, V> a[3],
+                                               Vec<T, V> b[3]) {
+    const T* A = side == 0 ? p.aE : p.aH;
+    const T* Bp = side == 0 ? p.bE : p.bH;
+#pragma unroll
+    for (int c = 0; c < 3; ++c) {
+        b[c] = coef_vec<T, V, CK>(Bp, p.cq[2 * side + 1], p.cs[8 * side + 4 + c], c * p.g.vol + o);
+        if constexpr (!UA) a[c] = coef_vec<T, V, CK>(A, p.cq[2 * side], p.cs[8 * side + c], c * p.g.vol + o);
+    }
+}
+
+template <typename T, int V, bool UA>
+__device__ __forceinline__ T alpha_of(const Vec<T, V>& a, T b, float a0, int c) {
+    if constexpr (UA) return b != T(0) ? T(1) : (T)a0;
+    return a.v[c];
+}
+
+// The roundings of the update, spelled out: which product of a sum of two the
+// compiler contracts into the FMA depends on the code around it.  These are
+// the ones the stream kernels compile to (Ex: fma(beta, curl, alpha E), the
+// other components fma(alpha, f, +-beta curl)), so both forms, a cell at a
+// time or 16 bytes, give the same bits.
+__device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
+__device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
+__device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
+__device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a, b); }
+
+// CPML of one axis at a thread's cells: psi <- air (b psi + c d) and the
+// corrections f1 += s1 b1 (ck d1 + psi1), f2 += s2 b2 (ck d2 + psi2) with
+// (s1, s2) = (-1, +1) when NEG1, else (+1, -1).  The axis is a template
+// argument and its two faces are picked by selects: a loop over the face
+// table with the axis read from it cost 436 instructions per warp on a box
+// with CPML all round.  SIDE: -1 picks the face by the coordinate; 0 and 1
+// are the two faces of an axis whose slabs overlap.
+template <typename T, int V, int A, int SIDE, bool NEG1>
+__device__ __forceinline__ void axis_psi(const AxisSlabs& x, int b, int i, int j, int k, const T d1[V], const T d2[V],
+                                         const Vec<T, V>& b1, const Vec<T, V>& b2, Vec<T, V>& f1, Vec<T, V>& f2) {
+    // V entries with one layer (x, y), or cell by cell along z
+    constexpr int NC = A == 2 ? V : 1, W = A == 2 ? 1 : V;
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
+        const int c = A == 0 ? i : (A == 1 ? j : k + m);
+        const bool hi = SIDE < 0 ? c >= x.lo1 : SIDE == 1;
+        const int l = hi ? c - x.lo1 : c, n = hi ? x.n[1] : x.n[0];
+        if ((unsigned)l >= (unsigned)n) continue;
+        const int s = (A == 0 ? l : i) * (hi ? x.s0[1] : x.s0[0]) + (A == 1 ? l : j) * (hi ? x.s1[1] : x.s1[0]) +
+                      (A == 2 ? l : k);
+        const unsigned slab = hi ? x.slab[1] : x.slab[0];
+        T* q = static_cast<T*>(hi ? x.psi[1] : x.psi[0]) + (size_t)(unsigned)b * (hi ? x.set[1] : x.set[0]) + s;
+        Vec<T, W> p1 = ldv<W>(q), p2 = ldv<W>(q + slab);
+        const T* __restrict__ t = static_cast<const T*>(hi ? x.bcc[1] : x.bcc[0]) + l;
+        const T cb = __ldg(t), cc = __ldg(t + n), ck = __ldg(t + 2 * n);
+        const unsigned char* air = hi ? x.air[1] : x.air[0];
+#pragma unroll
+        for (int w = 0; w < W; ++w) {
+            p1.v[w] = fma_(cc, d1[m + w], mul_(p1.v[w], cb));
+            p2.v[w] = fma_(cc, d2[m + w], mul_(p2.v[w], cb));
+            if (air) {
+                if (!air[s + w]) p1.v[w] = T(0);
+                if (!air[slab + s + w]) p2.v[w] = T(0);
+            }
+            const T c1 = fma_(ck, d1[m + w], p1.v[w]), c2 = fma_(ck, d2[m + w], p2.v[w]);
+            f1.v[m + w] = fma_(NEG1 ? -b1.v[m + w] : b1.v[m + w], c1, f1.v[m + w]);
+            f2.v[m + w] = fma_(NEG1 ? b2.v[m + w] : -b2.v[m + w], c2, f2.v[m + w]);
+        }
+        stv<W>(q, p1);
+        stv<W>(q + slab, p2);
+    }
+}
+
+// The CPML corrections of a thread's cells, x, y, z faces in that order.
+// E side: Ey += x, Ez -= x; Ex -= y, Ez += y; Ex += z, Ey -= z; the H side the
+// other way round.  dab: difference along axis a of component b; zs: the
+// thread's cells may lie in a z slab (uniform per warp).
+template <typename T, int V, int SIDE, bool E>
+__device__ __forceinline__ void cell_psi(const DirectArgs& d, int b, int i, int j, int k, bool zs,
+                                         const Vec<T, V> bc[3], const T dxz[V], const T dxy[V], const T dyz[V],
+                                         const T dyx[V], const T dzy[V], const T dzx[V], Vec<T, V>& fx, Vec<T, V>& fy,
+                                         Vec<T, V>& fz) {
+    axis_psi<T, V, 0, SIDE, !E>(d.ax[0], b, i, j, k, dxz, dxy, bc[1], bc[2], fy, fz);
+    axis_psi<T, V, 1, SIDE, E>(d.ax[1], b, i, j, k, dyz, dyx, bc[0], bc[2], fx, fz);
+    if (zs) axis_psi<T, V, 2, SIDE, !E>(d.ax[2], b, i, j, k, dzy, dzx, bc[0], bc[1], fx, fy);
+}
+
+// Row pads beyond k = nz stay +0 whatever their neighbours hold.
+template <typename T, int V>
+__device__ __forceinline__ void keep_pad(Vec<T, V>& f, int k, int nz) {
+#pragma unroll
+    for (int c = 1; c < V; ++c)
+        if (k + c > nz) f.v[c] = T(0);
+}
+
+// Row j, first cell k and z-slab flag of thread t of a plane: the vectors
+// clear of the z slabs of every row first, then (from a warp boundary on) the
+// others, so that only warps full of z-slab cells run that part.  False: no
+// cell.
+__device__ __forceinline__ bool direct_cell(const DirectArgs& d, int ny, unsigned t, int V, int& j, int& k, bool& zs) {
+    zs = t >= d.mid_threads;
+    if (!zs) {
+        j = (int)(__umulhi(2 * t, d.mid_div.m) >> d.mid_div.s);
+        k = (d.n_low + (int)t - j * d.n_mid) * V;
+    } else {
+        if (d.n_edge == 0) return false;  // the last block's spare threads
+        t -= d.mid_threads;
+        j = (int)(__umulhi(2 * t, d.edge_div.m) >> d.edge_div.s);
+        const int e = (int)t - j * d.n_edge;
+        k = (e < d.n_low ? e : e + d.n_mid) * V;
+    }
+    return j <= ny;
+}
+
+// Resident CTAs per SM asked of the compiler: 128 registers for the vector
+// form, 64 (float) and 85 (double) for one cell per thread.  Measured with the
+// vector form at 97 x 104 x 89 / 251 x 187 x 233 / 81 x 75 x 90 float64 (us
+// per step): 4 CTAs of 128 threads 31.7 / 215 / 28.7, 5 of 128 (102
+// registers) 32.6 / 216 / 31.0, 2 of 256 33.6 / 224 / 29.9, 3 of 256 (85
+// registers, spills) 36.3 / 228 / 35.3.
+template <typename T, int V>
+constexpr int direct_min_ctas() {
+    return V == 1 ? (sizeof(T) == 4 ? 8 : 6) : 4;
+}
+
+template <typename T, int V, int CK, bool UA, bool OV>
+__global__ void __launch_bounds__(kDirectThreads, direct_min_ctas<T, V>())
+    k_update_E(const __grid_constant__ StencilArgs<T> p, const __grid_constant__ DirectArgs d) {
     const Geom& g = p.g;
-    const int k = blockIdx.x * kBX + threadIdx.x;
-    const int j = blockIdx.y * kBY + threadIdx.y;
-    if (k > g.nz || j > g.ny) return;
-    const int i0 = blockIdx.z * p.ichunk;
-    const int i1 = min(i0 + p.ichunk, g.nx + 1);
+    int j, k;
+    bool zs;
+    if (!direct_cell(d, g.ny, blockIdx.x * blockDim.x + threadIdx.x, V, j, k, zs)) return;
     const long long vol = g.vol;
-    const long long si = g.si, sj = g.sj;
-    for (int i = i0; i < i1; ++i) {
-        const long long o = pidx(g, i, j, k);
-        const T aex = p.aE[o], aey = p.aE[vol + o], aez = p.aE[2 * vol + o];
-        const T bex = p.bE[o], bey = p.bE[vol + o], bez = p.bE[2 * vol + o];
-        for (int b = 0; b < p.B; ++b) {
-            T* E = p.e + (long long)b * 3 * vol;
-            const T* H = p.h + (long long)b * 3 * vol;
-            const T* Hx = H;
-            const T* Hy = H + vol;
-            const T* Hz = H + 2 * vol;
-            const T hx = Hx[o], hy = Hy[o], hz = Hz[o];
-            const T hz_jm = Hz[o - sj], hy_km = Hy[o - 1];
-            const T hx_km = Hx[o - 1], hz_im = Hz[o - si];
-            const T hy_im = Hy[o - si], hx_jm = Hx[o - sj];
-            // Same accumulation order as the reference kernels.
-            const T cx = ((hz - hz_jm) - hy) + hy_km;
-            const T cy = ((hx - hx_km) - hz) + hz_im;
-            const T cz = ((hy - hy_im) - hx) + hx_jm;
-            T ex = aex * E[o] + bex * cx;
-            T ey = aey * E[vol + o] + bey * cy;
-            T ez = aez * E[2 * vol + o] + bez * cz;
-            for (int fi = 0; fi < p.nfaces; ++fi) {
-                const FaceDev& f = p.f[fi];
-                const int coord = (f.axis == 0) ? i : ((f.axis == 1) ? j : k);
-                const int l = coord - f.lo;
-                if ((unsigned)l >= (unsigned)f.n) continue;
-                const long long s = slab_index<T>(f, l, i, j, k);
-                const T* bcc = static_cast<const T*>(f.bcc);
-                const T cb = bcc[l], cc = bcc[f.n + l], cck = bcc[2 * f.n + l];
-                T* psi = static_cast<T*>(f.psi) + (long long)b * 4 * f.slab;
-                T d1, d2;
-                if (f.axis == 0) {
-                    d1 = hz - hz_im;  // psi_Ey, Ey +=
-                    d2 = hy - hy_im;  // psi_Ez, Ez -=
-                } else if (f.axis == 1) {
-                    d1 = hz - hz_jm;  // psi_Ex, Ex -=
-                    d2 = hx - hx_jm;  // psi_Ez, Ez +=
-                } else {
-                    d1 = hy - hy_km;  // psi_Ex, Ex +=
-                    d2 = hx - hx_km;  // psi_Ey, Ey -=
-                }
-                T p1 = psi[s] * cb;
-                p1 = p1 + cc * d1;
-                if (!f.air[s]) p1 = T(0);
-                psi[s] = p1;
-                T p2 = psi[f.slab + s] * cb;
-                p2 = p2 + cc * d2;
-                if (!f.air[f.slab + s]) p2 = T(0);
-                psi[f.slab + s] = p2;
-                if (f.axis == 0) {
-                    ey = ey + bey * (cck * d1 + p1);
-                    ez = ez - bez * (cck * d2 + p2);
-                } else if (f.axis == 1) {
-                    ex = ex - bex * (cck * d1 + p1);
-                    ez = ez + bez * (cck * d2 + p2);
-                } else {
-                    ex = ex + bex * (cck * d1 + p1);
-                    ey = ey - bey * (cck * d2 + p2);
+    const int si = (int)g.si, sj = (int)g.sj;
+    const int i0 = blockIdx.y * d.np, i1 = min(i0 + d.np, g.nx + 1);
+    for (int b = threadIdx.y; b < p.B; b += blockDim.y) {
+        T* E = p.e + (long long)b * 3 * vol;
+        const T* __restrict__ H = p.h + (long long)b * 3 * vol;
+        int o = (int)pidx(g, i0, j, k);  // offset within a component: below 2^31 on any GPU this fits
+        Vec<T, V> hz_im = ldv<V>(H + 2 * vol + o - si), hy_im = ldv<V>(H + vol + o - si);
+        for (int i = i0; i < i1; ++i, o += si) {
+            Vec<T, V> a[3], bc[3];
+            load_cell_coef<T, V, CK, UA>(p, 0, o, a, bc);
+            const Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
+            const Vec<T, V> hz_jm = ldv<V>(H + 2 * vol + o - sj), hx_jm = ldv<V>(H + o - sj);
+            const T hy_km = H[vol + o - 1], hx_km = H[o - 1];
+            Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
+            T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const T hyk = c ? hy.v[c - (c > 0)] : hy_km, hxk = c ? hx.v[c - (c > 0)] : hx_km;
+                // Same accumulation order as the reference kernels.
+                const T cx = ((hz.v[c] - hz_jm.v[c]) - hy.v[c]) + hyk;
+                const T cy = ((hx.v[c] - hxk) - hz.v[c]) + hz_im.v[c];
+                const T cz = ((hy.v[c] - hy_im.v[c]) - hx.v[c]) + hx_jm.v[c];
+                ex.v[c] = fma_(bc[0].v[c], cx, mul_(alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[0], c), ex.v[c]));
+                ey.v[c] = fma_(alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[0], c), ey.v[c], mul_(bc[1].v[c], cy));
+                ez.v[c] = fma_(alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[0], c), ez.v[c], mul_(bc[2].v[c], cz));
+                dxz[c] = hz.v[c] - hz_im.v[c];
+                dxy[c] = hy.v[c] - hy_im.v[c];
+                dyz[c] = hz.v[c] - hz_jm.v[c];
+                dyx[c] = hx.v[c] - hx_jm.v[c];
+                dzy[c] = hy.v[c] - hyk;
+                dzx[c] = hx.v[c] - hxk;
+            }
+            cell_psi<T, V, OV ? 0 : -1, true>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
+            if constexpr (OV)
+                cell_psi<T, V, 1, true>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
+            // lumped ports of one edge: the thread that owns the edge steps
+            // the element on the value it is about to store
+            for (int q = 0; q < d.n_lumped; ++q) {
+                const int4 at = d.lumped[q];
+                if (at.x != i || at.y != j || (unsigned)(at.z - k) >= (unsigned)V) continue;
+#pragma unroll
+                for (int c = 0; c < V; ++c) {
+                    if (at.z != k + c) continue;
+                    const T v = lumped_edge_step<T>(d.ports[q], d.pa, b,
+                                                    at.w == 0 ? ex.v[c] : (at.w == 1 ? ey.v[c] : ez.v[c]));
+                    if (at.w == 0) ex.v[c] = v;
+                    if (at.w == 1) ey.v[c] = v;
+                    if (at.w == 2) ez.v[c] = v;
                 }
             }
-            E[o] = ex;
-            E[vol + o] = ey;
-            E[2 * vol + o] = ez;
+            if (k + V - 1 > g.nz) {
+                keep_pad(ex, k, g.nz);
+                keep_pad(ey, k, g.nz);
+                keep_pad(ez, k, g.nz);
+            }
+            stv<V>(E + o, ex);
+            stv<V>(E + vol + o, ey);
+            stv<V>(E + 2 * vol + o, ez);
+            hz_im = hz;
+            hy_im = hy;
         }
     }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(kBX* kBY) k_update_H(const StencilArgs<T> p) {
+template <typename T, int V, int CK, bool UA, bool OV>
+__global__ void __launch_bounds__(kDirectThreads, direct_min_ctas<T, V>())
+    k_update_H(const __grid_constant__ StencilArgs<T> p, const __grid_constant__ DirectArgs d) {
     const Geom& g = p.g;
-    const int k = blockIdx.x * kBX + threadIdx.x;
-    const int j = blockIdx.y * kBY + threadIdx.y;
-    if (k > g.nz || j > g.ny) return;
-    const int i0 = blockIdx.z * p.ichunk;
-    const int i1 = min(i0 + p.ichunk, g.nx + 1);
+    // the step counter, when nothing after this kernel reads it
+    if (d.advance && blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *d.advance += 1;
+    int j, k;
+    bool zs;
+    if (!direct_cell(d, g.ny, blockIdx.x * blockDim.x + threadIdx.x, V, j, k, zs)) return;
     const long long vol = g.vol;
-    const long long si = g.si, sj = g.sj;
-    for (int i = i0; i < i1; ++i) {
-        const long long o = pidx(g, i, j, k);
-        const T ahx = p.aH[o], ahy = p.aH[vol + o], ahz = p.aH[2 * vol + o];
-        const T bhx = p.bH[o], bhy = p.bH[vol + o], bhz = p.bH[2 * vol + o];
-        for (int b = 0; b < p.B; ++b) {
-            const T* E = p.e + (long long)b * 3 * vol;
-            T* H = p.h + (long long)b * 3 * vol;
-            const T* Ex = E;
-            const T* Ey = E + vol;
-            const T* Ez = E + 2 * vol;
-            const T ex = Ex[o], ey = Ey[o], ez = Ez[o];
-            const T ez_jp = Ez[o + sj], ey_kp = Ey[o + 1];
-            const T ex_kp = Ex[o + 1], ez_ip = Ez[o + si];
-            const T ey_ip = Ey[o + si], ex_jp = Ex[o + sj];
-            const T cx = ((ez_jp - ez) - ey_kp) + ey;
-            const T cy = ((ex_kp - ex) - ez_ip) + ez;
-            const T cz = ((ey_ip - ey) - ex_jp) + ex;
-            T hx = ahx * H[o] - bhx * cx;
-            T hy = ahy * H[vol + o] - bhy * cy;
-            T hz = ahz * H[2 * vol + o] - bhz * cz;
-            for (int fi = 0; fi < p.nfaces; ++fi) {
-                const FaceDev& f = p.f[fi];
-                const int coord = (f.axis == 0) ? i : ((f.axis == 1) ? j : k);
-                const int l = coord - f.lo;
-                if ((unsigned)l >= (unsigned)f.n) continue;
-                const long long s = slab_index<T>(f, l, i, j, k);
-                const T* bcc = static_cast<const T*>(f.bcc);
-                const T cb = bcc[l], cc = bcc[f.n + l], cck = bcc[2 * f.n + l];
-                T* psi = static_cast<T*>(f.psi) + (long long)b * 4 * f.slab;
-                T d1, d2;
-                if (f.axis == 0) {
-                    d1 = ez_ip - ez;  // psi_Hy, Hy -=
-                    d2 = ey_ip - ey;  // psi_Hz, Hz +=
-                } else if (f.axis == 1) {
-                    d1 = ez_jp - ez;  // psi_Hx, Hx +=
-                    d2 = ex_jp - ex;  // psi_Hz, Hz -=
-                } else {
-                    d1 = ey_kp - ey;  // psi_Hx, Hx -=
-                    d2 = ex_kp - ex;  // psi_Hy, Hy +=
-                }
-                const long long s1 = 2 * f.slab + s, s2 = 3 * f.slab + s;
-                T p1 = psi[s1] * cb;
-                p1 = p1 + cc * d1;
-                if (!f.air[s1]) p1 = T(0);
-                psi[s1] = p1;
-                T p2 = psi[s2] * cb;
-                p2 = p2 + cc * d2;
-                if (!f.air[s2]) p2 = T(0);
-                psi[s2] = p2;
-                if (f.axis == 0) {
-                    hy = hy - bhy * (cck * d1 + p1);
-                    hz = hz + bhz * (cck * d2 + p2);
-                } else if (f.axis == 1) {
-                    hx = hx + bhx * (cck * d1 + p1);
-                    hz = hz - bhz * (cck * d2 + p2);
-                } else {
-                    hx = hx - bhx * (cck * d1 + p1);
-                    hy = hy + bhy * (cck * d2 + p2);
-                }
+    const int si = (int)g.si, sj = (int)g.sj;
+    const int i0 = blockIdx.y * d.np, i1 = min(i0 + d.np, g.nx + 1);
+    for (int b = threadIdx.y; b < p.B; b += blockDim.y) {
+        T* H = p.h + (long long)b * 3 * vol;
+        const T* __restrict__ E = p.e + (long long)b * 3 * vol;
+        int o = (int)pidx(g, i1 - 1, j, k);
+        Vec<T, V> ez_ip = ldv<V>(E + 2 * vol + o + si), ey_ip = ldv<V>(E + vol + o + si);
+        for (int i = i1 - 1; i >= i0; --i, o -= si) {
+            Vec<T, V> a[3], bc[3];
+            load_cell_coef<T, V, CK, UA>(p, 1, o, a, bc);
+            const Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
+            const Vec<T, V> ez_jp = ldv<V>(E + 2 * vol + o + sj), ex_jp = ldv<V>(E + o + sj);
+            const T ey_kp = E[vol + o + V], ex_kp = E[o + V];
+            Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
+            T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
+#pragma unroll
+            for (int c = 0; c < V; ++c) {
+                const T eyk = c < V - 1 ? ey.v[(c + 1) % V] : ey_kp, exk = c < V - 1 ? ex.v[(c + 1) % V] : ex_kp;
+                const T cx = ((ez_jp.v[c] - ez.v[c]) - eyk) + ey.v[c];
+                const T cy = ((exk - ex.v[c]) - ez_ip.v[c]) + ez.v[c];
+                const T cz = ((ey_ip.v[c] - ey.v[c]) - ex_jp.v[c]) + ex.v[c];
+                hx.v[c] = fma_(alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[1], c), hx.v[c], -mul_(bc[0].v[c], cx));
+                hy.v[c] = fma_(alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[1], c), hy.v[c], -mul_(bc[1].v[c], cy));
+                hz.v[c] = fma_(alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[1], c), hz.v[c], -mul_(bc[2].v[c], cz));
+                dxz[c] = ez_ip.v[c] - ez.v[c];
+                dxy[c] = ey_ip.v[c] - ey.v[c];
+                dyz[c] = ez_jp.v[c] - ez.v[c];
+                dyx[c] = ex_jp.v[c] - ex.v[c];
+                dzy[c] = eyk - ey.v[c];
+                dzx[c] = exk - ex.v[c];
             }
-            H[o] = hx;
-            H[vol + o] = hy;
-            H[2 * vol + o] = hz;
+            cell_psi<T, V, OV ? 0 : -1, false>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
+            if constexpr (OV)
+                cell_psi<T, V, 1, false>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
+            if (k + V - 1 > g.nz) {
+                keep_pad(hx, k, g.nz);
+                keep_pad(hy, k, g.nz);
+                keep_pad(hz, k, g.nz);
+            }
+            stv<V>(H + o, hx);
+            stv<V>(H + vol + o, hy);
+            stv<V>(H + 2 * vol + o, hz);
+            ez_ip = ez;
+            ey_ip = ey;
         }
     }
+}
+
+// bits 0 / 1 of flags[side]: some entry has alpha != (beta != 0) / alpha != 1
+// (so an unset bit 0 means alpha follows from beta with a0 = 0, an unset
+// bit 1 with a0 = 1); over the entries of the component's own sub-box.
+template <typename T, int CK>
+__global__ void __launch_bounds__(256) k_unit_alpha(const StencilArgs<T> p, int* flags) {
+    const Geom& g = p.g;
+    const int side = blockIdx.y / 3, c = blockIdx.y % 3;
+    int ni, nj, nk;
+    comp_shape(g, 3 * side + c, ni, nj, nk);
+    const T* __restrict__ A = side == 0 ? p.aE : p.aH;
+    const T* __restrict__ Bp = side == 0 ? p.bE : p.bH;
+    int bad = 0;
+    for (long long row = blockIdx.x; row < (long long)ni * nj; row += gridDim.x) {
+        const long long o = c * g.vol + pidx(g, (int)(row / nj), (int)(row % nj), 0);
+        for (int k = threadIdx.x; k < nk; k += blockDim.x) {
+            const T b = coef_at<T, CK>(Bp, p.cq[2 * side + 1], p.cs[8 * side + 4 + c], o + k);
+            const T a = coef_at<T, CK>(A, p.cq[2 * side], p.cs[8 * side + c], o + k);
+            if (a != (b != T(0) ? T(1) : T(0))) bad |= 1;
+            if (a != T(1)) bad |= 2;
+        }
+    }
+    if (bad) atomicOr(flags + side, bad);
 }
 
 template <typename T>
@@ -253,20 +456,106 @@ __global__ void k_energy_final(const double* __restrict__ partials, int n, doubl
 
 }  // namespace
 
+// t / n for t < 2^31 as mulhi(2 t, m) >> s.
+static DirectDiv direct_div(int n) {
+    int s = 0;
+    while ((1u << s) < (unsigned)n) ++s;
+    return {(unsigned)(((1ull << (31 + s)) / (unsigned)n) + 1), s};
+}
+
+// Grid of the direct kernels: V cells and np planes per thread, 128 threads,
+// the field sets of a cell in threadIdx.y (as many as there are warps).  which: 0 = E,
+// 1 = H.  Returns whether both faces of an axis reach one cell.
 template <typename T>
-void launch_update_E(const StencilArgs<T>& a, cudaStream_t s) {
-    dim3 block(kBX, kBY, 1);
-    dim3 grid((a.g.nz + 1 + kBX - 1) / kBX, (a.g.ny + 1 + kBY - 1) / kBY,
-              (a.g.nx + 1 + a.ichunk - 1) / a.ichunk);
-    k_update_E<T><<<grid, block, 0, s>>>(a);
+static bool direct_grid(const StencilArgs<T>& a, DirectArgs& d, int V, int which, dim3& grid, dim3& block) {
+    for (auto& x : d.ax) x = AxisSlabs{};
+    for (auto& x : d.ax) x.lo1 = 0x7fffffff;
+    for (int q = 0; q < a.nfaces; ++q) {
+        const FaceDev& f = a.f[q];
+        AxisSlabs& x = d.ax[f.axis];
+        const int hi = f.lo > 0 || x.n[0] > 0 ? 1 : 0;  // a face of the whole axis first, then the far side
+        if (hi) x.lo1 = f.lo;
+        x.n[hi] = f.n;
+        x.s0[hi] = f.dJ * f.pk;
+        x.s1[hi] = f.pk;
+        x.slab[hi] = (unsigned)f.slab;
+        x.set[hi] = 4 * f.slab;
+        x.psi[hi] = static_cast<T*>(f.psi) + 2 * which * f.slab;  // E1, E2 or H1, H2
+        x.bcc[hi] = f.bcc;
+        x.air[hi] = f.masked ? f.air + 2 * which * f.slab : nullptr;
+    }
+    bool overlap = false;
+    for (const AxisSlabs& x : d.ax) overlap = overlap || x.n[0] > x.lo1;
+    const int nset = std::min(a.B, kDirectThreads / 32);
+    block = dim3(kDirectThreads / nset / 32 * 32, nset, 1);
+    if (d.np < 1) d.np = 1;
+    const int nvec = a.g.nz / V + 1;
+    d.n_low = std::min(nvec, (d.ax[2].n[0] + V - 1) / V);
+    const int high = d.ax[2].n[1] > 0 ? nvec - std::min(nvec, d.ax[2].lo1 / V) : 0;
+    d.n_mid = std::max(0, nvec - d.n_low - high);
+    d.n_edge = nvec - d.n_mid;
+    const long long rows = a.g.ny + 1;
+    d.mid_threads = (unsigned)((rows * d.n_mid + 31) / 32 * 32);
+    d.mid_div = direct_div(std::max(1, d.n_mid));
+    d.edge_div = direct_div(std::max(1, d.n_edge));
+    grid = dim3((unsigned)((d.mid_threads + rows * d.n_edge + block.x - 1) / block.x),
+                (unsigned)((a.g.nx + d.np) / d.np), 1);
+    return overlap;
+}
+
+template <typename T, int V, int CK>
+static void direct_launch(const StencilArgs<T>& a, DirectArgs d, int which, cudaStream_t s) {
+    dim3 grid, block;
+    const bool overlap = direct_grid<T>(a, d, V, which, grid, block);
+    // alpha read from memory: conductive or mixed coefficients, and small
+    // meshes whose thick slabs overlap
+    const auto go = [&](auto kE, auto kH) {
+        if (which == 0)
+            kE<<<grid, block, 0, s>>>(a, d);
+        else
+            kH<<<grid, block, 0, s>>>(a, d);
+    };
+    if (overlap)
+        go(k_update_E<T, V, CK, false, true>, k_update_H<T, V, CK, false, true>);
+    else if (a.unit_alpha)
+        go(k_update_E<T, V, CK, true, false>, k_update_H<T, V, CK, true, false>);
+    else
+        go(k_update_E<T, V, CK, false, false>, k_update_H<T, V, CK, false, false>);
+}
+
+// Meshes up to this many cells take one cell per thread: their step is the
+// latency of one short thread.  Measured, one cell against 16 bytes per
+// thread (us per step): 7.6 / 9.4 at 10 thousand cells, 8.5 / 11.5 at 100
+// thousand, 12.8 / 13.5 at 262 thousand, 18.5 / 18.3 at 512 thousand; four
+// field sets of 164 thousand cells 24.3 / 20.6.  The cells alone decide, not
+// the batch, so that a field set's bits do not depend on its batch.
+constexpr long long kScalarCells = 150000;
+
+template <typename T>
+void launch_direct_half(const StencilArgs<T>& a, const DirectArgs& d, int which, cudaStream_t s) {
+    constexpr int W = 16 / (int)sizeof(T);
+    const bool one = (long long)(a.g.nx + 1) * (a.g.ny + 1) * (a.g.nz + 1) <= kScalarCells;
+    const auto kind = [&](auto ck) {
+        constexpr int CK = decltype(ck)::value;
+        one ? direct_launch<T, 1, CK>(a, d, which, s) : direct_launch<T, W, CK>(a, d, which, s);
+    };
+    if (a.coef_kind == kCoefF16)
+        kind(std::integral_constant<int, kCoefF16>());
+    else if (a.coef_kind == kCoefBF16)
+        kind(std::integral_constant<int, kCoefBF16>());
+    else
+        kind(std::integral_constant<int, kCoefNative>());
 }
 
 template <typename T>
-void launch_update_H(const StencilArgs<T>& a, cudaStream_t s) {
-    dim3 block(kBX, kBY, 1);
-    dim3 grid((a.g.nz + 1 + kBX - 1) / kBX, (a.g.ny + 1 + kBY - 1) / kBY,
-              (a.g.nx + 1 + a.ichunk - 1) / a.ichunk);
-    k_update_H<T><<<grid, block, 0, s>>>(a);
+void launch_unit_alpha(const StencilArgs<T>& a, int* flags, cudaStream_t s) {
+    const dim3 grid(592, 6);
+    if (a.coef_kind == kCoefF16)
+        k_unit_alpha<T, kCoefF16><<<grid, 256, 0, s>>>(a, flags);
+    else if (a.coef_kind == kCoefBF16)
+        k_unit_alpha<T, kCoefBF16><<<grid, 256, 0, s>>>(a, flags);
+    else
+        k_unit_alpha<T, kCoefNative><<<grid, 256, 0, s>>>(a, flags);
 }
 
 template <typename T>
@@ -294,8 +583,8 @@ void launch_energy(const T* e, const T* h, const T* meps, const T* mmu, const Ge
 }
 
 #define FITB_INST(T)                                                                           \
-    template void launch_update_E<T>(const StencilArgs<T>&, cudaStream_t);                    \
-    template void launch_update_H<T>(const StencilArgs<T>&, cudaStream_t);                    \
+    template void launch_direct_half<T>(const StencilArgs<T>&, const DirectArgs&, int, cudaStream_t); \
+    template void launch_unit_alpha<T>(const StencilArgs<T>&, int*, cudaStream_t);             \
     template void launch_pack<T>(const T*, T*, const Geom&, int, long long, cudaStream_t);     \
     template void launch_unpack<T>(const T*, T*, const Geom&, int, long long, cudaStream_t);   \
     template void launch_energy<T>(const T*, const T*, const T*, const T*, const Geom&, int,    \

@@ -1,0 +1,118 @@
+"""The direct stencil kernels (a handle's own choice of form) against the
+stream kernels, which share none of their code: at the remainders of their
+16-byte cells and of a plane's threads, on both sides of the one-cell-per-thread
+bound, with slabs that overlap, masked or missing, for every way alpha can
+relate to beta, batch widths around a block's warps and the compact storages."""
+
+from __future__ import annotations
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+STEPS = 37  # odd, more than one 32-slot monitor block
+TOL = {"double": 1e-12, "single": 1e-5}  # relative to the largest field
+
+
+def _problem(n, layers, alpha, batch, seed=3):
+    from magnelio_b200 import host
+    from magnelio_b200.problem import FACES, CpmlFace, DftMonitor, FitProblem, LumpedPort
+
+    rng = np.random.default_rng(seed)
+    nx, ny, nz = n
+    d = [1e-3 * rng.uniform(0.8, 1.2, v) for v in n]
+    x, y, z = (np.concatenate([[0.0], np.cumsum(v)]) for v in d)
+    mat = rng.integers(0, 3, n).astype(np.int32)
+    M_eps = host.build_M_eps(x, y, z, [1.0, 2.5, 6.0], mat)
+    M_mu = host.build_M_mu(x, y, z)
+    dt = host.courant_dt(x, y, z)
+    aE, bE, aH, bH = host.leapfrog_coefficients(M_eps, M_mu, dt)
+    frozen = rng.choice(aE.size, aE.size // 50, replace=False)
+    bE[frozen] = 0.0
+    if alpha == "pec":  # frozen at zero: alpha = (beta != 0)
+        aE[frozen] = 0.0
+    elif alpha == "mixed":  # some frozen at zero, some kept: alpha is read
+        aE[frozen[::2]] = 0.0
+    elif alpha == "lossy":
+        aE[bE != 0] *= rng.uniform(0.9, 1.0, int(np.sum(bE != 0)))
+    prob = FitProblem(nx=nx, ny=ny, nz=nz, dt=dt, dx=d[0], dy=d[1], dz=d[2], alpha_E=aE, beta_E=bE, alpha_H=aH,
+                      beta_H=bH, M_eps=M_eps, M_mu=M_mu, batch=batch)
+    for face, k in zip(FACES, layers):
+        if not k:
+            continue
+        axis = "xyz".index(face[0])
+        b, c, ck = host.cpml_tables(d[axis], face, dt, thickness_cells=k)
+        air = (None,) * 4
+        if face == "ymin":  # PEC inside one slab
+            shapes = [((nx, k, nz + 1)), (nx + 1, k, nz), (nx + 1, k, nz), (nx, k, nz + 1)]
+            air = tuple((rng.random(s) > 0.2).astype(np.uint8) for s in shapes)
+        prob.cpml.append(CpmlFace(face, b, c, ck, air))
+    ey0 = nx * (ny + 1) * (nz + 1)
+    for p in range(2):
+        i, j, k = nx // 2, ny // 2, (nz // 2 + p) % nz
+        flat = ey0 + (i * ny + j) * (nz + 1) + k
+        prob.lumped.append(LumpedPort(np.array([flat]), np.ones(1), np.array([dt / M_eps[flat]]), R=50.0,
+                                      v_src=[rng.standard_normal(STEPS) for _ in range(batch)]))
+    prob.monitors.append(DftMonitor(((0, nx), (0, ny), (nz // 2, nz // 2 + 1)), ("Ex", "Hz"), np.array([1e9, 5e9]), 1))
+    prob.e0 = [rng.standard_normal(aE.size) * (aE != 0) for _ in range(batch)]
+    prob.h0 = [rng.standard_normal(aH.size) / 377.0 for _ in range(batch)]
+    return prob
+
+
+def _march(prob, precision, form, coef):
+    with prob.build_engine(precision) as eng:
+        if form:
+            eng.configure_stencil(form)
+        if coef != "native":
+            eng.set_coefficient_storage(coef)
+        eng.step(STEPS)
+        return ([eng.read_fields(b) for b in range(prob.batch)], [eng.read_vi(b) for b in range(prob.batch)],
+                [eng.read_dft(0, c) for c in ("Ex", "Hz")])
+
+
+@pytest.mark.parametrize("n,layers,alpha,batch,precision,coef", [
+    ((5, 4, 1), (0, 0, 0, 0, 0, 0), "pec", 1, "double", "native"),           # one cell in z, no slab
+    ((9, 7, 12), (3, 3, 2, 2, 8, 7), "one", 1, "double", "native"),          # overlapping z slabs
+    ((8, 9, 11), (8, 5, 9, 9, 0, 4), "pec", 2, "double", "native"),          # slabs as thick as the axis
+    ((20, 19, 31), (4, 4, 4, 4, 4, 4), "mixed", 3, "single", "native"),      # batch without a stream form
+    ((53, 52, 54), (6, 5, 4, 7, 5, 6), "pec", 1, "single", "native"),        # just below the 16-byte bound
+    ((53, 53, 55), (6, 5, 4, 7, 5, 6), "one", 1, "single", "native"),        # just above it
+    ((54, 53, 56), (0, 0, 6, 6, 1, 3), "lossy", 1, "single", "native"),      # z remainders 1 and 3
+    ((62, 51, 49), (5, 0, 0, 5, 49, 0), "one", 1, "double", "native"),       # a z slab of the whole axis
+    ((62, 51, 50), (5, 5, 0, 0, 30, 30), "pec", 1, "double", "native"),      # overlapping, 16-byte form
+    ((300, 23, 25), (10, 10, 2, 2, 6, 6), "one", 5, "single", "native"),     # more field sets than warps
+    ((53, 53, 55), (6, 6, 6, 6, 6, 6), "pec", 2, "single", "f16"),
+    ((53, 53, 55), (6, 6, 6, 6, 6, 6), "one", 1, "single", "bf16"),
+    ((53, 53, 55), (6, 6, 6, 6, 6, 6), "pec", 1, "double", "f16"),
+])
+def test_direct_kernels_match_the_stream_kernels(n, layers, alpha, batch, precision, coef):
+    prob = _problem(n, layers, alpha, batch)
+    got = _march(prob, precision, None, coef)
+    if batch in (1, 2, 4, 8, 16):
+        want = _march(prob, precision, "stream", coef)
+    else:  # one field set per handle
+        want = ([], [], None)
+        for b in range(batch):
+            one = _problem(n, layers, alpha, batch)
+            one.batch, one.e0, one.h0 = 1, [one.e0[b]], [one.h0[b]]
+            for lp in one.lumped:
+                lp.v_src = [lp.v_src[b]]
+            f, vi, dft = _march(one, precision, "stream", coef)
+            want[0].append(f[0])
+            want[1].append(vi[0])
+            want = (want[0], want[1], want[2] or dft)
+    tol = TOL[precision]
+
+    def close(a, b, scale, t):
+        assert np.all(np.isfinite(a)) and float(np.max(np.abs(a - b))) <= t * scale
+
+    for q in range(2):
+        scale = max(float(np.max(np.abs(f[q]))) for f in want[0])
+        for a, b in zip(got[0], want[0]):
+            close(a[q], b[q], scale, tol)
+        scale = max(float(np.max(np.abs(v[q]))) for v in want[1])
+        for a, b in zip(got[1], want[1]):
+            close(a[q], b[q], scale, 10 * tol)
+    for a, b in zip(got[2], want[2]):
+        close(a, b, float(np.max(np.abs(b))), 1e-5)  # float32 bins
