@@ -412,6 +412,8 @@ int fitb_add_dft_monitor(fitb_handle* h, const fitb_dft_desc* d, int32_t* out_id
  * (n_freq, ni, nj, nk); re / im arrays of that many doubles. */
 int fitb_read_dft(fitb_handle* h, int32_t mon, int32_t b, int32_t comp,
                   double* re, double* im, size_t count);
+/* The same bins as (re, im) pairs: 2 count doubles, a complex128 array. */
+int fitb_read_dft_complex(fitb_handle* h, int32_t mon, int32_t b, int32_t comp, double* bins, size_t count);
 
 /* ---- time stepping -------------------------------------------------- */
 /* Advance all field sets by n_steps leapfrog steps (the body of the loop

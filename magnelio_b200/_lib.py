@@ -179,6 +179,7 @@ SIGNATURES = {
     "fitb_set_modal_source": ([vp, i32, i32, i32, i64, P_f64], C.c_int),
     "fitb_add_dft_monitor": ([vp, C.POINTER(FitbDftDesc), P_i32], C.c_int),
     "fitb_read_dft": ([vp, i32, i32, i32, P_f64, P_f64, sz], C.c_int),
+    "fitb_read_dft_complex": ([vp, i32, i32, i32, P_f64, sz], C.c_int),
     "fitb_step": ([vp, i64], C.c_int),
     "fitb_sync": ([vp], C.c_int),
     "fitb_query": ([vp, C.POINTER(C.c_int32)], C.c_int),

@@ -26,6 +26,7 @@
 
 #include "../../include/fitb200.h"
 #include "direct.cuh"
+#include "hostcopy.cuh"
 
 namespace fitb {
 
@@ -308,6 +309,7 @@ struct Handle {
     StreamPlan splan{};
     DevBuf status;
     HostBuf host_io;  // pinned landing area of fitb_read_vi
+    HostLanes lanes;  // of the field and monitor reads
     // Compact coefficient storage of the stream kernels (kCoefF16 /
     // kCoefBF16): {aE, bE, aH, bH} as 16-bit [3][vol] with power-of-two
     // scales cs[4 * array + component]; coef_max holds the per-component
@@ -430,8 +432,15 @@ void unpack3(Handle& H, const T* dev_padded, T* host_flat, int c0) {
         off += H.comp_size(c0 + q);
     }
     ck(cudaGetLastError(), "unpack");
-    ck(cudaMemcpyAsync(host_flat, H.staging.p, (size_t)n * sizeof(T), cudaMemcpyDeviceToHost, H.stream),
-       "D2H staging");
+    const size_t bytes = (size_t)n * sizeof(T);
+    if (bytes <= HostLanes::kSmall) {
+        ck(cudaMemcpyAsync(host_flat, H.staging.p, bytes, cudaMemcpyDeviceToHost, H.stream), "D2H staging");
+    } else {
+        char* dst = reinterpret_cast<char*>(host_flat);
+        ck(H.lanes.read(H.desc.device, H.staging.p, bytes, H.stream,
+                        [dst](size_t off, const void* p, size_t m) { memcpy(dst + off, p, m); }),
+           "D2H staging");
+    }
     ck(cudaStreamSynchronize(H.stream), "unpack sync");
     check_device_status(H);
 }
@@ -2929,9 +2938,7 @@ int fitb_add_dft_monitor(fitb_handle* h, const fitb_dft_desc* d, int32_t* out_id
     FITB_CATCH
 }
 
-int fitb_read_dft(fitb_handle* h, int32_t mon, int32_t b, int32_t comp, double* re, double* im, size_t count) {
-    FITB_TRY
-    Handle& H = H_of(h);
+static const float2* dft_bins(Handle& H, int32_t mon, int32_t b, int32_t comp, size_t count, bool null_out) {
     if (mon < 0 || mon >= (int)H.dft.size()) fail(FITB_ERR_ARG, "monitor %d does not exist", mon);
     if (b < 0 || b >= H.B) fail(FITB_ERR_ARG, "field set %d out of range", b);
     fitb::DftHost& m = *H.dft[mon];
@@ -2939,16 +2946,40 @@ int fitb_read_dft(fitb_handle* h, int32_t mon, int32_t b, int32_t comp, double* 
     for (int q = 0; q < m.dev.ncomp; ++q)
         if (m.dev.comps[q] == comp) ci = q;
     if (ci < 0) fail(FITB_ERR_ARG, "monitor %d does not record component %d", mon, comp);
-    size_t n = (size_t)m.dev.nf * m.dev.ncell;
-    if (count != n || !re || !im) fail(FITB_ERR_ARG, "expected %zu bins", n);
+    const size_t n = (size_t)m.dev.nf * m.dev.ncell;
+    if (count != n || null_out) fail(FITB_ERR_ARG, "expected %zu bins", n);
     fitb::dft_flush_pending(H);
-    std::vector<float2> bins(n);
-    size_t off = ((size_t)b * m.dev.ncomp + ci) * n;
-    ck(cudaMemcpy(bins.data(), m.bins.as<float2>() + off, n * sizeof(float2), cudaMemcpyDeviceToHost), "read bins");
-    for (size_t q = 0; q < n; ++q) {
-        re[q] = bins[q].x;
-        im[q] = bins[q].y;
-    }
+    return m.bins.as<float2>() + ((size_t)b * m.dev.ncomp + ci) * n;
+}
+
+int fitb_read_dft(fitb_handle* h, int32_t mon, int32_t b, int32_t comp, double* re, double* im, size_t count) {
+    FITB_TRY
+    Handle& H = H_of(h);
+    const float2* bins = dft_bins(H, mon, b, comp, count, !re || !im);
+    ck(H.lanes.read(H.desc.device, bins, count * sizeof(float2), H.stream,
+                    [re, im](size_t off, const void* p, size_t m) {
+                        const float2* v = static_cast<const float2*>(p);
+                        const size_t q0 = off / sizeof(float2);
+                        for (size_t q = 0; q < m / sizeof(float2); ++q) {
+                            re[q0 + q] = v[q].x;
+                            im[q0 + q] = v[q].y;
+                        }
+                    }),
+       "read bins");
+    FITB_CATCH
+}
+
+int fitb_read_dft_complex(fitb_handle* h, int32_t mon, int32_t b, int32_t comp, double* bins_out, size_t count) {
+    FITB_TRY
+    Handle& H = H_of(h);
+    const float2* bins = dft_bins(H, mon, b, comp, count, !bins_out);
+    ck(H.lanes.read(H.desc.device, bins, count * sizeof(float2), H.stream,
+                    [bins_out](size_t off, const void* p, size_t m) {
+                        const float* v = static_cast<const float*>(p);
+                        double* out = bins_out + off / sizeof(float);
+                        for (size_t q = 0; q < m / sizeof(float); ++q) out[q] = v[q];
+                    }),
+       "read bins");
     FITB_CATCH
 }
 

@@ -541,10 +541,10 @@ class FitEngine:
     def read_dft(self, mon: int, comp: str, b: int = 0) -> np.ndarray:
         _, shape, nf = self._monitors[mon]
         n = int(nf * np.prod(shape))
-        re = np.empty(n)
-        im = np.empty(n)
-        check(self._lib.fitb_read_dft(self._h, int(mon), int(b), COMPONENTS.index(comp), f64p(re), f64p(im), n))
-        return (re + 1j * im).reshape(nf, *shape)
+        out = np.empty((nf, *shape), dtype=np.complex128)
+        check(self._lib.fitb_read_dft_complex(self._h, int(mon), int(b), COMPONENTS.index(comp),
+                                              f64p(out.view(np.float64)), n))
+        return out
 
     # ---- stepping --------------------------------------------------------
     def step(self, n: int) -> None:

@@ -116,3 +116,32 @@ def test_direct_kernels_match_the_stream_kernels(n, layers, alpha, batch, precis
             close(a[q], b[q], scale, 10 * tol)
     for a, b in zip(got[2], want[2]):
         close(a, b, float(np.max(np.abs(b))), 1e-5)  # float32 bins
+
+
+@pytest.mark.parametrize("n", [(43, 41, 24), (44, 41, 24), (90, 67, 61), (131, 89, 113)])
+def test_large_reads_return_every_entry(n):
+    """Fields and monitor bins around the size of one piece of the threaded
+    read, and over many pieces with a ragged last one: what was set comes
+    back, and the complex read equals the split one."""
+    import ctypes as C
+
+    from magnelio_b200 import _lib
+    from magnelio_b200._lib import f64p
+    from magnelio_b200.engine import FitEngine
+
+    rng = np.random.default_rng(4)
+    d = [np.full(v, 1e-3) for v in n]
+    with FitEngine(*n, 1e-13) as eng:
+        one = [np.ones(s) for s in (eng.n_E, eng.n_E, eng.n_H, eng.n_H)]
+        eng.set_coefficients(one[0], 0.1 * one[1], one[2], 0.1 * one[3])
+        m = eng.add_dft_monitor(tuple((0, v) for v in n), ("Ey",), [1e9, 2e9, 3e9], *d)
+        e, h = (rng.standard_normal(s).astype(np.float32) for s in (eng.n_E, eng.n_H))
+        eng.set_fields(e, h)
+        ge, gh = eng.read_fields()
+        assert np.array_equal(ge, e) and np.array_equal(gh, h)
+        eng.step(2)
+        bins = eng.read_dft(m, "Ey")
+        re, im = np.empty(bins.size), np.empty(bins.size)
+        _lib.check(_lib.load().fitb_read_dft(eng._h, C.c_int32(m), 0, 1, f64p(re), f64p(im), bins.size))
+        assert np.array_equal(bins.real.ravel(), re) and np.array_equal(bins.imag.ravel(), im)
+        assert np.any(re != 0) and np.all(np.isfinite(re))
