@@ -14,8 +14,10 @@
 // storage, double operations).
 //
 // The reference applies the CPML corrections after this update
-// (fit_td.py:858-874): on a side with dispersion the stencil kernel runs
-// without its fused CPML and k_cpml_pass applies it face by face here.
+// (fit_td.py:858-874): on a side whose dispersive entries reach into a CPML
+// slab the stencil kernel runs without its fused CPML and k_cpml_pass applies
+// it face by face here.  Where no entry takes both, the orders agree and the
+// direct kernels keep the CPML fused.
 #include "fitb_common.cuh"
 
 namespace fitb {
@@ -55,24 +57,6 @@ __device__ __forceinline__ double j_hist(const DispDev& d, int b, long long s) {
 }
 
 template <typename T>
-__global__ void k_disp_subtract(T* F, long long blk, int B, const T* __restrict__ beta, const DispDev d) {
-    const long long work = (long long)d.n_unique * B;
-    for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < work;
-         q += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(q / d.n_unique);
-        const long long u = q - (long long)b * d.n_unique;
-        const long long o = d.uoff[u];
-        T v = F[b * blk + o];
-        const double bt = (double)beta[o];
-        for (int r = d.ustart[u]; r < d.ustart[u + 1]; ++r) {
-            const double jh = j_hist<T>(d, b, d.ustate[r]);
-            v = (T)__dsub_rn((double)v, __dmul_rn(bt, jh));
-        }
-        F[b * blk + o] = v;
-    }
-}
-
-template <typename T>
 __device__ __forceinline__ T sub_rn(T a, T b);
 template <>
 __device__ __forceinline__ float sub_rn<float>(float a, float b) { return __fsub_rn(a, b); }
@@ -85,31 +69,49 @@ __device__ __forceinline__ float mul_rn<float>(float a, float b) { return __fmul
 template <>
 __device__ __forceinline__ double mul_rn<double>(double a, double b) { return __dmul_rn(a, b); }
 
+// Pole states of state s from its entry's new value v.
 template <typename T>
-__global__ void k_disp_advance(const T* __restrict__ F, long long blk, int B, const DispDev d) {
-    const long long work = (long long)d.n_states * B;
+__device__ __forceinline__ void advance_poles(const DispDev& d, int b, long long s, T v) {
+    const T fp = static_cast<const T*>(d.fprev)[(long long)b * d.n_states + s];
+    const double g64 = (double)mul_rn<T>(static_cast<const T*>(d.g)[s], sub_rn<T>(v, fp));
+    const int bk = d.state_block[s];
+    const int q0 = d.pole_start[bk], q1 = d.pole_start[bk + 1];
+    T* J = static_cast<T*>(d.J) + (long long)b * d.n_slots + d.slot[s];
+    for (int p = q0; p < q1; ++p) {
+        T* js = J + 2 * (p - q0);
+        if (d.kind[p] == 0) {
+            js[0] = (T)__dadd_rn(__dmul_rn((double)js[0], d.k_re[p]), __dmul_rn(d.c_re[p], g64));
+        } else {
+            const double jr = (double)js[0], ji = (double)js[1];
+            const double mr = __dsub_rn(__dmul_rn(jr, d.k_re[p]), __dmul_rn(ji, d.k_im[p]));
+            const double mi = __dadd_rn(__dmul_rn(jr, d.k_im[p]), __dmul_rn(ji, d.k_re[p]));
+            js[0] = (T)__dadd_rn(mr, __dmul_rn(d.c_re[p], g64));
+            js[1] = (T)__dadd_rn(mi, __dmul_rn(d.c_im[p], g64));
+        }
+    }
+}
+
+// One thread per entry: the history currents of its states subtracted in
+// block order, then its states advanced from the corrected value (a state
+// belongs to one entry, so nothing is shared between threads and one launch
+// does both; the launches, not the bytes, bound this on ordinary meshes).
+template <typename T>
+__global__ void k_disp_update(T* F, long long blk, int B, const T* __restrict__ beta, const DispDev d) {
+    const long long work = (long long)d.n_unique * B;
     for (long long q = blockIdx.x * (long long)blockDim.x + threadIdx.x; q < work;
          q += (long long)gridDim.x * blockDim.x) {
-        const int b = (int)(q / d.n_states);
-        const long long s = q - (long long)b * d.n_states;
-        const T fp = static_cast<const T*>(d.fprev)[q];
-        const T gd = mul_rn<T>(static_cast<const T*>(d.g)[s], sub_rn<T>(F[b * blk + d.off[s]], fp));
-        const double g64 = (double)gd;
-        const int bk = d.state_block[s];
-        const int q0 = d.pole_start[bk], q1 = d.pole_start[bk + 1];
-        T* J = static_cast<T*>(d.J) + (long long)b * d.n_slots + d.slot[s];
-        for (int p = q0; p < q1; ++p) {
-            T* js = J + 2 * (p - q0);
-            if (d.kind[p] == 0) {
-                js[0] = (T)__dadd_rn(__dmul_rn((double)js[0], d.k_re[p]), __dmul_rn(d.c_re[p], g64));
-            } else {
-                const double jr = (double)js[0], ji = (double)js[1];
-                const double mr = __dsub_rn(__dmul_rn(jr, d.k_re[p]), __dmul_rn(ji, d.k_im[p]));
-                const double mi = __dadd_rn(__dmul_rn(jr, d.k_im[p]), __dmul_rn(ji, d.k_re[p]));
-                js[0] = (T)__dadd_rn(mr, __dmul_rn(d.c_re[p], g64));
-                js[1] = (T)__dadd_rn(mi, __dmul_rn(d.c_im[p], g64));
-            }
+        const int b = (int)(q / d.n_unique);
+        const long long u = q - (long long)b * d.n_unique;
+        const long long o = d.uoff[u];
+        T v = F[b * blk + o];
+        const double bt = (double)beta[o];
+        const int r0 = d.ustart[u], r1 = d.ustart[u + 1];
+        for (int r = r0; r < r1; ++r) {
+            const double jh = j_hist<T>(d, b, d.ustate[r]);
+            v = (T)__dsub_rn((double)v, __dmul_rn(bt, jh));
         }
+        F[b * blk + o] = v;
+        for (int r = r0; r < r1; ++r) advance_poles<T>(d, b, d.ustate[r], v);
     }
 }
 
@@ -212,8 +214,7 @@ void launch_disp_save(const T* F, long long blk, int B, const DispDev& d, cudaSt
 template <typename T>
 void launch_disp_update(T* F, long long blk, int B, const T* beta, const DispDev& d, cudaStream_t s) {
     if (d.n_states <= 0) return;
-    k_disp_subtract<T><<<grid_for(d.n_unique * B), 256, 0, s>>>(F, blk, B, beta, d);
-    k_disp_advance<T><<<grid_for(d.n_states * B), 256, 0, s>>>(F, blk, B, d);
+    k_disp_update<T><<<grid_for(d.n_unique * B), 256, 0, s>>>(F, blk, B, beta, d);
 }
 template <typename T>
 void launch_cpml_pass(const StencilArgs<T>& a, int q, int side, cudaStream_t s) {

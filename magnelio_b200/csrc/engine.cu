@@ -261,6 +261,7 @@ struct Handle {
     std::vector<std::unique_ptr<DftHost>> dft;
     std::vector<std::unique_ptr<PlaneWaveHost>> pws;
     DispHost disp[2];  // E side, H side
+    bool disp_clear[2] = {false, false};  // the side's dispersive entries lie outside the CPML slabs
     SibcHost sibc;     // surface-impedance walls (H side)
     std::vector<std::unique_ptr<BandHost>> band;  // band-subspace DTBC ports
     DevBuf d_band;
@@ -591,6 +592,26 @@ void build_fix_cells(Handle& H) {
 
 void build_slab_units(Handle& H);
 
+// Whether no dispersive state lies in a CPML slab.  The slab step applies
+// the CPML inside its kernel, before the ADE update of the same side; the
+// reference applies the ADE update first (fit_td.py:833-874), so the two
+// orders agree exactly when no entry takes both.
+bool side_clear_of_cpml(const Handle& H, int side) {
+    for (long long off : H.disp[side].off) {
+        const long long r = off % H.g.vol;
+        const int i = (int)(r / H.g.si) - 2;
+        const long long rr = r % H.g.si;
+        const int j = (int)(rr / H.g.sj), k = (int)(rr % H.g.sj);
+        for (auto& f : H.faces) {
+            const int c = f->dev.axis == 0 ? i : (f->dev.axis == 1 ? j : k);
+            if (c >= f->dev.lo && c < f->dev.lo + f->dev.n) return false;
+        }
+    }
+    return true;
+}
+
+bool disp_clear_of_cpml(const Handle& H) { return side_clear_of_cpml(H, 0) && side_clear_of_cpml(H, 1); }
+
 // The lumped ports may step inside the direct E kernel when each has one edge
 // of its own and nothing else touches that edge between the E update and the
 // ports: no plane wave, ADE or band port on the E side, and no modal port that
@@ -627,6 +648,7 @@ void refresh_port_tables(Handle& H) {
     for (auto& lp : H.lumped) ld.push_back(lp->dev);
     upload(H.d_lumped, ld);
     find_lumped_in_E(H);
+    for (int sd = 0; sd < 2; ++sd) H.disp_clear[sd] = side_clear_of_cpml(H, sd);
     std::vector<ModalDev> md;
     for (auto& mp : H.modal) {
         ModalDev d = mp->dev;
@@ -835,25 +857,6 @@ bool tile_skip_on(const Handle& H) {
     return !(e && std::string(e) == "0") && H.pws.empty() && !H.disp[0].present() && !H.disp[1].present();
 }
 
-// Whether no dispersive state lies in a CPML slab.  The slab step applies
-// the CPML inside its kernel, before the ADE update of the same side; the
-// reference applies the ADE update first (fit_td.py:833-874), so the two
-// orders agree exactly when no entry takes both.
-bool disp_clear_of_cpml(const Handle& H) {
-    for (const DispHost& D : H.disp)
-        for (long long off : D.off) {
-            const long long r = off % H.g.vol;
-            const int i = (int)(r / H.g.si) - 2;
-            const long long rr = r % H.g.si;
-            const int j = (int)(rr / H.g.sj), k = (int)(rr % H.g.sj);
-            for (auto& f : H.faces) {
-                const int c = f->dev.axis == 0 ? i : (f->dev.axis == 1 ? j : k);
-                if (c >= f->dev.lo && c < f->dev.lo + f->dev.n) return false;
-            }
-        }
-    return true;
-}
-
 void build_slab_units(Handle& H) {
     if ((H.disp[0].present() || H.disp[1].present()) && !disp_clear_of_cpml(H))
         fail(FITB_ERR_STATE, "the slab step takes dispersive materials only outside the CPML slabs");
@@ -954,13 +957,24 @@ void plan_stencil(Handle& H) {
 // the bulk-copy pipeline on request, the batched kernel for B > 1.  A side
 // with dispersive materials takes its CPML corrections in separate passes
 // after the ADE update, so its stencil launch carries no faces.
+// Whether a side's CPML runs as passes after its ADE / SIBC update instead of
+// inside the stencil kernel.  The direct kernels keep it where no dispersive
+// entry lies in a slab: each entry then takes the same operations in the same
+// order either way.  (The passes read the native coefficients, so a compact
+// storage keeps them.)
+bool cpml_as_passes(const Handle& H, int side) {
+    if (side == 1 && H.sibc.present()) return true;
+    if (!H.disp[side].present()) return false;
+    return !(H.stencil_mode == kModeSimple && H.coef_kind == kCoefNative && H.disp_clear[side]);
+}
+
 // In a step of the direct kernels, pa != null, the E launch steps the lumped
 // ports it can (H.lumped_in_E) and the H launch advances the step counter
 // when `advance` says so.
 template <typename T>
 void launch_half(Handle& H, int which, const PortsArgs* pa = nullptr, bool advance = false) {
     StencilArgs<T> sa = stencil_args<T>(H);
-    if (H.disp[which].present() || (which == 1 && H.sibc.present())) sa.nfaces = 0;
+    if (cpml_as_passes(H, which)) sa.nfaces = 0;
     switch (H.stencil_mode) {
         case kModeStream:
             launch_stream_half<T>(sa, H.splan, H.stream_variant, which, H.stream);
@@ -1067,13 +1081,14 @@ int disp_complete(Handle& H, int sd) {
     int n = 0;
     if (H.disp[sd].present()) {
         launch_disp_update<T>(F, H.e_block(), H.B, beta, H.disp[sd].dev, H.stream);
-        n += 2;
+        ++n;
     }
     // the SIBC walls after the mu-side ADE (fit_td.py:903-914)
     if (sibc) {
         launch_sibc_update<T>(F, H.e_block(), H.B, beta, H.sibc.dev, H.stream);
         n += 2;
     }
+    if (!cpml_as_passes(H, sd)) return n;
     StencilArgs<T> sa = stencil_args<T>(H);
     for (int q = 0; q < sa.nfaces; ++q) {
         launch_cpml_pass<T>(sa, q, sd, H.stream);
@@ -1124,7 +1139,7 @@ int enqueue_step_fused(Handle& H) {
         // E-side ADE after the curl update and the CPML (which never share
         // an entry with it, disp_clear_of_cpml), before the ports
         launch_disp_update<T>(e_new, H.e_block(), H.B, H.bE.as<T>(), H.disp[0].dev, H.stream);
-        n += 2;
+        ++n;
     }
     for (auto& pw : H.pws) {
         launch_plane_wave<T>(e_new, H.e_block(), H.B, pw->dev, 0, H.step.as<long long>(), H.stream);
@@ -1151,7 +1166,7 @@ int enqueue_step_fused(Handle& H) {
     }
     if (H.disp[1].present()) {
         launch_disp_update<T>(h_new, H.e_block(), H.B, H.bH.as<T>(), H.disp[1].dev, H.stream);
-        n += 2;
+        ++n;
     }
     for (auto& pw : H.pws) {
         launch_plane_wave<T>(h_new, H.e_block(), H.B, pw->dev, 1, H.step.as<long long>(), H.stream);
@@ -2154,6 +2169,7 @@ int fitb_add_cpml(fitb_handle* h, int32_t face, int32_t n_pml, const double* b, 
         fitb::add_cpml_impl<float>(H, face, n_pml, b, c, ck_, air);
     else
         fitb::add_cpml_impl<double>(H, face, n_pml, b, c, ck_, air);
+    H.port_tables_dirty = true;  // plans that depend on the slabs
     fitb::invalidate_graphs(H);
     FITB_CATCH
 }

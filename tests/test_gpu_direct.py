@@ -145,3 +145,23 @@ def test_large_reads_return_every_entry(n):
         _lib.check(_lib.load().fitb_read_dft(eng._h, C.c_int32(m), 0, 1, f64p(re), f64p(im), bins.size))
         assert np.array_equal(bins.real.ravel(), re) and np.array_equal(bins.imag.ravel(), im)
         assert np.any(re != 0) and np.all(np.isfinite(re))
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("n,layers", [((26, 24, 45), 4), ((58, 55, 61), 6)])
+def test_cpml_stays_fused_beside_clear_dispersion(n, layers, precision):
+    """Dispersive entries outside the slabs: the direct kernels keep the CPML
+    fused, the stream kernels run it as passes after the ADE update."""
+    from magnelio_b200.workloads import dispersive_slab
+
+    prob = dispersive_slab(*n, seed=6, cpml_cells=layers, n_freq=3)
+    out = []
+    for form in (None, "stream"):
+        with prob.build_engine(precision) as eng:
+            if form:
+                eng.configure_stencil(form)
+            eng.step(3 * max(n))
+            out.append((*eng.read_fields(), *(eng.read_dft(m, "Ex") for m in range(2))))
+    for q, (a, b) in enumerate(zip(*out)):
+        scale = float(np.max(np.abs(b)))
+        assert scale > 0 and float(np.max(np.abs(a - b))) <= (TOL[precision] if q < 2 else 1e-5) * scale
