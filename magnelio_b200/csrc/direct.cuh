@@ -21,7 +21,8 @@ struct AxisSlabs {
     int n[2], s0[2], s1[2];
     unsigned slab[2];
     size_t set[2];
-    void* psi[2];
+    const void* psi[2];
+    void* psi_out[2];
     const void* bcc[2];
     const unsigned char* air[2];
 };
@@ -36,7 +37,9 @@ struct DirectArgs {
     int n_low, n_mid, n_edge;
     unsigned mid_threads;
     DirectDiv mid_div, edge_div;
-    AxisSlabs ax[3];
+    AxisSlabs ax[2][3];  // E side, H side
+    int ping_pong;       // the new fields and psi go to the *_next buffers
+    int slab_bits;       // E with the slab step's roundings
     int n_lumped;
     int4 lumped[kDirectLumped];
     const LumpedDev* ports;

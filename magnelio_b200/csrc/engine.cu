@@ -297,6 +297,7 @@ struct Handle {
     int unit_alpha = 0;
     float a0[2] = {};
     DevBuf scan;  // flags of the coefficient scan
+    int slab_ichunk = 0;  // march depth the caller gave the fused form (0: none)
     // lumped ports that step inside the direct E kernel (all or none)
     bool lumped_in_E = false;
     int4 lumped_cell[kDirectLumped] = {};
@@ -957,6 +958,13 @@ void plan_stencil(Handle& H) {
 // the bulk-copy pipeline on request, the batched kernel for B > 1.  A side
 // with dispersive materials takes its CPML corrections in separate passes
 // after the ADE update, so its stencil launch carries no faces.
+void direct_ports(Handle& H, const PortsArgs& pa, DirectArgs& da) {
+    da.n_lumped = (int)H.lumped.size();
+    for (int q = 0; q < da.n_lumped; ++q) da.lumped[q] = H.lumped_cell[q];
+    da.ports = H.d_lumped.as<LumpedDev>();
+    da.pa = pa;
+}
+
 // Whether a side's CPML runs as passes after its ADE / SIBC update instead of
 // inside the stencil kernel.  The direct kernels keep it where no dispersive
 // entry lies in a slab: each entry then takes the same operations in the same
@@ -966,6 +974,29 @@ bool cpml_as_passes(const Handle& H, int side) {
     if (side == 1 && H.sibc.present()) return true;
     if (!H.disp[side].present()) return false;
     return !(H.stencil_mode == kModeSimple && H.coef_kind == kCoefNative && H.disp_clear[side]);
+}
+
+// The slab step (fused 16-25) on the direct kernels.  They are faster than
+// its unit lists at every size measured (float32, CPML all round, us per
+// step, lists / direct: 60 / 23 at 0.9 M cells, 280 / 200 at 10.9 M, 415 /
+// 310 at 16.8 M, 1119 / 840 at 49 M), with the same bits.  The lists stay
+// where the caller gave a march depth, and where more than kDeadShare of the
+// units are dead, which the lists leave out (a cross junction with 808 of
+// 1200 units dead steps on its lists at 84 Gcell/s of the dense mesh; the
+// direct kernels reach 56).
+constexpr double kDeadShare = 0.3;
+bool slab_on_lists(const Handle& H) {
+    if (H.slab_ichunk > 0) return true;
+    int units = H.n_slab_dead;
+    for (int n : H.n_slab_units) units += n;
+    return H.n_slab_dead > kDeadShare * units;
+}
+// In place, in the current buffer set, where nothing stands between the E and
+// the H update but lumped ports that step inside the E kernel; else from one
+// buffer set to the other, with the H cells beside the ports recomputed.
+bool slab_in_place(const Handle& H) {
+    return H.stencil_mode == kModeFused && is_slab_variant(H.fused_variant) && !slab_on_lists(H) && H.pws.empty() &&
+           H.modal.empty() && !H.disp[0].present() && !H.disp[1].present() && (H.lumped.empty() || H.lumped_in_E);
 }
 
 // In a step of the direct kernels, pa != null, the E launch steps the lumped
@@ -988,13 +1019,11 @@ void launch_half(Handle& H, int which, const PortsArgs* pa = nullptr, bool advan
             break;
         default: {
             DirectArgs da{};
-            da.np = H.direct_np;
-            if (pa && which == 0 && H.lumped_in_E) {
-                da.n_lumped = (int)H.lumped.size();
-                for (int q = 0; q < da.n_lumped; ++q) da.lumped[q] = H.lumped_cell[q];
-                da.ports = H.d_lumped.as<LumpedDev>();
-                da.pa = *pa;
-            }
+            if (H.stencil_mode == kModeFused)
+                da.slab_bits = 1;  // the slab step in place
+            else
+                da.np = H.direct_np;
+            if (pa && which == 0 && H.lumped_in_E) direct_ports(H, *pa, da);
             if (advance) da.advance = H.step.as<long long>();
             launch_direct_half<T>(sa, da, which, H.stream);
         }
@@ -1008,6 +1037,14 @@ void launch_half(Handle& H, int which, const PortsArgs* pa = nullptr, bool advan
 template <typename T>
 int launch_fused(Handle& H, const StencilArgs<T>& sa) {
     if (is_slab_variant(H.fused_variant)) {
+        if (!slab_on_lists(H)) {
+            DirectArgs da{};
+            da.slab_bits = 1;
+            da.ping_pong = slab_in_place(H) ? 0 : 1;
+            launch_direct_half<T>(sa, da, 0, H.stream);
+            launch_direct_half<T>(sa, da, 1, H.stream);
+            return 2;
+        }
         const int4* units[kSlabLists];
         bool air = false;
         for (int q = 0; q < kSlabLists; ++q) units[q] = H.slab_units[q].as<int4>();
@@ -1187,7 +1224,7 @@ int enqueue_step_fused(Handle& H) {
 
 template <typename T>
 int enqueue_step(Handle& H) {
-    if (H.stencil_mode == kModeFused) return enqueue_step_fused<T>(H);
+    if (H.stencil_mode == kModeFused && !slab_in_place(H)) return enqueue_step_fused<T>(H);
     // in-place kernels below
     int n = 0;
     PortsArgs pa = ports_args(H);
@@ -1219,7 +1256,7 @@ int enqueue_step(Handle& H) {
                        (int)((H.cap + kConvChunk - 1) / kConvChunk), H.stream);
         n += 2;
     }
-    const bool direct = H.stencil_mode == kModeSimple;
+    const bool direct = H.stencil_mode == kModeSimple || H.stencil_mode == kModeFused;
     if (!H.lumped.empty() && !(direct && H.lumped_in_E)) {
         launch_lumped<T>(H.Ec().as<T>(), pa, H.d_lumped.as<LumpedDev>(), (int)H.lumped.size(), H.stream);
         ++n;
@@ -1281,7 +1318,7 @@ cudaGraphExec_t capture(Handle& H, int nsteps, int* launches_per) {
 // expired and the step's results are not valid.
 // the stencil forms whose copy pipelines record a status word
 bool has_device_status(const Handle& H) {
-    return H.stencil_mode == kModeBulk || (H.stencil_mode == kModeFused && H.fused_variant >= kFusedTileBase);
+    return H.stencil_mode == kModeBulk ||  (H.stencil_mode == kModeFused && H.fused_variant >= kFusedTileBase);
 }
 
 // error out on a nonzero status word `st` (read after the step), resetting it
@@ -1367,7 +1404,7 @@ void run_steps(Handle& H, long long nsteps) {
     per = H.launches_per_step;
     if (nsteps == 0) return;
     long long left = nsteps;
-    const bool swaps = H.stencil_mode == kModeFused;
+    const bool swaps = H.stencil_mode == kModeFused && !slab_in_place(H);
     while (left >= H.chunk) {
         ck(cudaGraphLaunch(H.graph_chunk[H.cur], H.stream), "graph launch");
         if (swaps && (H.chunk & 1)) H.cur ^= 1;
@@ -1459,7 +1496,7 @@ void set_form(Handle& H, int kind, int variant, int ichunk) {
     if (kind == kModeVec) H.vec_variant = variant;
     if (kind == kModeStream) H.stream_variant = compact ? 0 : variant;
     H.stencil_mode = kind;
-    H.direct_np = ichunk;
+    H.direct_np = H.slab_ichunk = ichunk;
     plan_stencil(H);
     if (ichunk > 0) {
         const int nplanes = H.g.nx + 1;
@@ -3051,7 +3088,7 @@ int fitb_time_stencil(fitb_handle* h, int32_t n_iter, double* ms_e, double* ms_h
         int nl = 0;
         for (int q = 0; q < n2; ++q) {
             nl += fitb::launch_fused_any(H);
-            H.cur ^= 1;
+            if (!fitb::slab_in_place(H)) H.cur ^= 1;
         }
         ck(cudaEventRecord(ev[1], H.stream), "event record");
         ck(cudaEventSynchronize(ev[1]), "event sync");

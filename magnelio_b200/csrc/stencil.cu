@@ -150,36 +150,56 @@ __device__ __forceinline__ double mul_(double a, double b) { return __dmul_rn(a,
 template <typename T, int V, int A, int SIDE, bool NEG1>
 __device__ __forceinline__ void axis_psi(const AxisSlabs& x, int b, int i, int j, int k, const T d1[V], const T d2[V],
                                          const Vec<T, V>& b1, const Vec<T, V>& b2, Vec<T, V>& f1, Vec<T, V>& f2) {
-    // V entries with one layer (x, y), or cell by cell along z
+    // V entries with one layer (x, y), or cell by cell along z: there
+    // the psi loads of all the cells go out before the first is used
     constexpr int NC = A == 2 ? V : 1, W = A == 2 ? 1 : V;
+    Vec<T, W> p1[NC], p2[NC];
+    bool on[NC];
+    bool any = false;
 #pragma unroll
     for (int m = 0; m < NC; ++m) {
         const int c = A == 0 ? i : (A == 1 ? j : k + m);
         const bool hi = SIDE < 0 ? c >= x.lo1 : SIDE == 1;
         const int l = hi ? c - x.lo1 : c, n = hi ? x.n[1] : x.n[0];
-        if ((unsigned)l >= (unsigned)n) continue;
+        on[m] = (unsigned)l < (unsigned)n;
+        any = any || on[m];
+        if (!on[m]) continue;
         const int s = (A == 0 ? l : i) * (hi ? x.s0[1] : x.s0[0]) + (A == 1 ? l : j) * (hi ? x.s1[1] : x.s1[0]) +
                       (A == 2 ? l : k);
-        const unsigned slab = hi ? x.slab[1] : x.slab[0];
-        T* q = static_cast<T*>(hi ? x.psi[1] : x.psi[0]) + (size_t)(unsigned)b * (hi ? x.set[1] : x.set[0]) + s;
-        Vec<T, W> p1 = ldv<W>(q), p2 = ldv<W>(q + slab);
+        const T* q = static_cast<const T*>(hi ? x.psi[1] : x.psi[0]) +
+                     ((size_t)(unsigned)b * (hi ? x.set[1] : x.set[0]) + s);
+        p1[m] = ldv<W>(q);
+        p2[m] = ldv<W>(q + (hi ? x.slab[1] : x.slab[0]));
+    }
+    if (!any) return;
+#pragma unroll
+    for (int m = 0; m < NC; ++m) {
+        if (!on[m]) continue;
+        const int c = A == 0 ? i : (A == 1 ? j : k + m);
+        const bool hi = SIDE < 0 ? c >= x.lo1 : SIDE == 1;
+        const int l = hi ? c - x.lo1 : c, n = hi ? x.n[1] : x.n[0];
+        const int s = (A == 0 ? l : i) * (hi ? x.s0[1] : x.s0[0]) + (A == 1 ? l : j) * (hi ? x.s1[1] : x.s1[0]) +
+                      (A == 2 ? l : k);
         const T* __restrict__ t = static_cast<const T*>(hi ? x.bcc[1] : x.bcc[0]) + l;
         const T cb = __ldg(t), cc = __ldg(t + n), ck = __ldg(t + 2 * n);
+        const unsigned slab = hi ? x.slab[1] : x.slab[0];
         const unsigned char* air = hi ? x.air[1] : x.air[0];
 #pragma unroll
         for (int w = 0; w < W; ++w) {
-            p1.v[w] = fma_(cc, d1[m + w], mul_(p1.v[w], cb));
-            p2.v[w] = fma_(cc, d2[m + w], mul_(p2.v[w], cb));
+            p1[m].v[w] = fma_(cc, d1[m + w], mul_(p1[m].v[w], cb));
+            p2[m].v[w] = fma_(cc, d2[m + w], mul_(p2[m].v[w], cb));
             if (air) {
-                if (!air[s + w]) p1.v[w] = T(0);
-                if (!air[slab + s + w]) p2.v[w] = T(0);
+                if (!air[s + w]) p1[m].v[w] = T(0);
+                if (!air[slab + s + w]) p2[m].v[w] = T(0);
             }
-            const T c1 = fma_(ck, d1[m + w], p1.v[w]), c2 = fma_(ck, d2[m + w], p2.v[w]);
+            const T c1 = fma_(ck, d1[m + w], p1[m].v[w]), c2 = fma_(ck, d2[m + w], p2[m].v[w]);
             f1.v[m + w] = fma_(NEG1 ? -b1.v[m + w] : b1.v[m + w], c1, f1.v[m + w]);
             f2.v[m + w] = fma_(NEG1 ? b2.v[m + w] : -b2.v[m + w], c2, f2.v[m + w]);
         }
-        stv<W>(q, p1);
-        stv<W>(q + slab, p2);
+        T* out = static_cast<T*>(hi ? x.psi_out[1] : x.psi_out[0]) +
+                 ((size_t)(unsigned)b * (hi ? x.set[1] : x.set[0]) + s);
+        stv<W>(out, p1[m]);
+        stv<W>(out + slab, p2[m]);
     }
 }
 
@@ -188,13 +208,13 @@ __device__ __forceinline__ void axis_psi(const AxisSlabs& x, int b, int i, int j
 // other way round.  dab: difference along axis a of component b; zs: the
 // thread's cells may lie in a z slab (uniform per warp).
 template <typename T, int V, int SIDE, bool E>
-__device__ __forceinline__ void cell_psi(const DirectArgs& d, int b, int i, int j, int k, bool zs,
+__device__ __forceinline__ void cell_psi(const AxisSlabs ax[3], int b, int i, int j, int k, bool zs,
                                          const Vec<T, V> bc[3], const T dxz[V], const T dxy[V], const T dyz[V],
                                          const T dyx[V], const T dzy[V], const T dzx[V], Vec<T, V>& fx, Vec<T, V>& fy,
                                          Vec<T, V>& fz) {
-    axis_psi<T, V, 0, SIDE, !E>(d.ax[0], b, i, j, k, dxz, dxy, bc[1], bc[2], fy, fz);
-    axis_psi<T, V, 1, SIDE, E>(d.ax[1], b, i, j, k, dyz, dyx, bc[0], bc[2], fx, fz);
-    if (zs) axis_psi<T, V, 2, SIDE, !E>(d.ax[2], b, i, j, k, dzy, dzx, bc[0], bc[1], fx, fy);
+    axis_psi<T, V, 0, SIDE, !E>(ax[0], b, i, j, k, dxz, dxy, bc[1], bc[2], fy, fz);
+    axis_psi<T, V, 1, SIDE, E>(ax[1], b, i, j, k, dyz, dyx, bc[0], bc[2], fx, fz);
+    if (zs) axis_psi<T, V, 2, SIDE, !E>(ax[2], b, i, j, k, dzy, dzx, bc[0], bc[1], fx, fy);
 }
 
 // Row pads beyond k = nz stay +0 whatever their neighbours hold.
@@ -235,7 +255,119 @@ constexpr int direct_min_ctas() {
     return V == 1 ? (sizeof(T) == 4 ? 8 : 6) : 4;
 }
 
+// E_new of a thread's cells at plane i of field set b.  hz_im, hy_im: H of
+// plane i - 1; on return H of plane i.  ES: the roundings of the slab step (all
+// components fma(beta, curl, alpha E)) instead of the stream kernels'.
+template <typename T, int V, int CK, bool UA, bool OV, bool ES>
+__device__ __forceinline__ void cell_E(const StencilArgs<T>& p, const DirectArgs& d, const T* E, const T* H, T* Eo,
+                                       int b, int i, int j, int k, int o, bool zs, Vec<T, V>& hz_im,
+                                       Vec<T, V>& hy_im) {
+    const Geom& g = p.g;
+    const long long vol = g.vol;
+    const int sj = (int)g.sj;
+    Vec<T, V> a[3], bc[3];
+    load_cell_coef<T, V, CK, UA>(p, 0, o, a, bc);
+    const Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
+    const Vec<T, V> hz_jm = ldv<V>(H + 2 * vol + o - sj), hx_jm = ldv<V>(H + o - sj);
+    const T hy_km = H[vol + o - 1], hx_km = H[o - 1];
+    Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
+    T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const T hyk = c ? hy.v[c - (c > 0)] : hy_km, hxk = c ? hx.v[c - (c > 0)] : hx_km;
+        // Same accumulation order as the reference kernels.
+        const T cx = ((hz.v[c] - hz_jm.v[c]) - hy.v[c]) + hyk;
+        const T cy = ((hx.v[c] - hxk) - hz.v[c]) + hz_im.v[c];
+        const T cz = ((hy.v[c] - hy_im.v[c]) - hx.v[c]) + hx_jm.v[c];
+        const T ax = alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[0], c);
+        const T ay = alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[0], c);
+        const T az = alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[0], c);
+        ex.v[c] = fma_(bc[0].v[c], cx, mul_(ax, ex.v[c]));
+        ey.v[c] = ES ? fma_(bc[1].v[c], cy, mul_(ay, ey.v[c])) : fma_(ay, ey.v[c], mul_(bc[1].v[c], cy));
+        ez.v[c] = ES ? fma_(bc[2].v[c], cz, mul_(az, ez.v[c])) : fma_(az, ez.v[c], mul_(bc[2].v[c], cz));
+        dxz[c] = hz.v[c] - hz_im.v[c];
+        dxy[c] = hy.v[c] - hy_im.v[c];
+        dyz[c] = hz.v[c] - hz_jm.v[c];
+        dyx[c] = hx.v[c] - hx_jm.v[c];
+        dzy[c] = hy.v[c] - hyk;
+        dzx[c] = hx.v[c] - hxk;
+    }
+    cell_psi<T, V, OV ? 0 : -1, true>(d.ax[0], b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
+    if constexpr (OV) cell_psi<T, V, 1, true>(d.ax[0], b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
+    // lumped ports of one edge: the thread that owns the edge steps the
+    // element on the value it is about to store
+    for (int q = 0; q < d.n_lumped; ++q) {
+        const int4 at = d.lumped[q];
+        if (at.x != i || at.y != j || (unsigned)(at.z - k) >= (unsigned)V) continue;
+#pragma unroll
+        for (int c = 0; c < V; ++c) {
+            if (at.z != k + c) continue;
+            const T v =
+                lumped_edge_step<T>(d.ports[q], d.pa, b, at.w == 0 ? ex.v[c] : (at.w == 1 ? ey.v[c] : ez.v[c]));
+            if (at.w == 0) ex.v[c] = v;
+            if (at.w == 1) ey.v[c] = v;
+            if (at.w == 2) ez.v[c] = v;
+        }
+    }
+    if (k + V - 1 > g.nz) {
+        keep_pad(ex, k, g.nz);
+        keep_pad(ey, k, g.nz);
+        keep_pad(ez, k, g.nz);
+    }
+    stv<V>(Eo + o, ex);
+    stv<V>(Eo + vol + o, ey);
+    stv<V>(Eo + 2 * vol + o, ez);
+    hz_im = hz;
+    hy_im = hy;
+}
+
+// H_new of a thread's cells at plane i from E_new.  ez_ip, ey_ip: E of plane
+// i + 1; on return E of plane i.
 template <typename T, int V, int CK, bool UA, bool OV>
+__device__ __forceinline__ void cell_H(const StencilArgs<T>& p, const DirectArgs& d, const T* E, const T* H, T* Ho,
+                                       int b, int i, int j, int k, int o, bool zs, Vec<T, V>& ez_ip,
+                                       Vec<T, V>& ey_ip) {
+    const Geom& g = p.g;
+    const long long vol = g.vol;
+    const int sj = (int)g.sj;
+    Vec<T, V> a[3], bc[3];
+    load_cell_coef<T, V, CK, UA>(p, 1, o, a, bc);
+    const Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
+    const Vec<T, V> ez_jp = ldv<V>(E + 2 * vol + o + sj), ex_jp = ldv<V>(E + o + sj);
+    const T ey_kp = E[vol + o + V], ex_kp = E[o + V];
+    Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
+    T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
+#pragma unroll
+    for (int c = 0; c < V; ++c) {
+        const T eyk = c < V - 1 ? ey.v[(c + 1) % V] : ey_kp, exk = c < V - 1 ? ex.v[(c + 1) % V] : ex_kp;
+        const T cx = ((ez_jp.v[c] - ez.v[c]) - eyk) + ey.v[c];
+        const T cy = ((exk - ex.v[c]) - ez_ip.v[c]) + ez.v[c];
+        const T cz = ((ey_ip.v[c] - ey.v[c]) - ex_jp.v[c]) + ex.v[c];
+        hx.v[c] = fma_(alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[1], c), hx.v[c], -mul_(bc[0].v[c], cx));
+        hy.v[c] = fma_(alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[1], c), hy.v[c], -mul_(bc[1].v[c], cy));
+        hz.v[c] = fma_(alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[1], c), hz.v[c], -mul_(bc[2].v[c], cz));
+        dxz[c] = ez_ip.v[c] - ez.v[c];
+        dxy[c] = ey_ip.v[c] - ey.v[c];
+        dyz[c] = ez_jp.v[c] - ez.v[c];
+        dyx[c] = ex_jp.v[c] - ex.v[c];
+        dzy[c] = eyk - ey.v[c];
+        dzx[c] = exk - ex.v[c];
+    }
+    cell_psi<T, V, OV ? 0 : -1, false>(d.ax[1], b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
+    if constexpr (OV) cell_psi<T, V, 1, false>(d.ax[1], b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
+    if (k + V - 1 > g.nz) {
+        keep_pad(hx, k, g.nz);
+        keep_pad(hy, k, g.nz);
+        keep_pad(hz, k, g.nz);
+    }
+    stv<V>(Ho + o, hx);
+    stv<V>(Ho + vol + o, hy);
+    stv<V>(Ho + 2 * vol + o, hz);
+    ez_ip = ez;
+    ey_ip = ey;
+}
+
+template <typename T, int V, int CK, bool UA, bool OV, bool ES>
 __global__ void __launch_bounds__(kDirectThreads, direct_min_ctas<T, V>())
     k_update_E(const __grid_constant__ StencilArgs<T> p, const __grid_constant__ DirectArgs d) {
     const Geom& g = p.g;
@@ -243,67 +375,15 @@ __global__ void __launch_bounds__(kDirectThreads, direct_min_ctas<T, V>())
     bool zs;
     if (!direct_cell(d, g.ny, blockIdx.x * blockDim.x + threadIdx.x, V, j, k, zs)) return;
     const long long vol = g.vol;
-    const int si = (int)g.si, sj = (int)g.sj;
+    const int si = (int)g.si;
     const int i0 = blockIdx.y * d.np, i1 = min(i0 + d.np, g.nx + 1);
     for (int b = threadIdx.y; b < p.B; b += blockDim.y) {
-        T* E = p.e + (long long)b * 3 * vol;
-        const T* __restrict__ H = p.h + (long long)b * 3 * vol;
+        const long long fs = (long long)b * 3 * vol;
+        const T* H = p.h + fs;
         int o = (int)pidx(g, i0, j, k);  // offset within a component: below 2^31 on any GPU this fits
         Vec<T, V> hz_im = ldv<V>(H + 2 * vol + o - si), hy_im = ldv<V>(H + vol + o - si);
-        for (int i = i0; i < i1; ++i, o += si) {
-            Vec<T, V> a[3], bc[3];
-            load_cell_coef<T, V, CK, UA>(p, 0, o, a, bc);
-            const Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
-            const Vec<T, V> hz_jm = ldv<V>(H + 2 * vol + o - sj), hx_jm = ldv<V>(H + o - sj);
-            const T hy_km = H[vol + o - 1], hx_km = H[o - 1];
-            Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
-            T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
-#pragma unroll
-            for (int c = 0; c < V; ++c) {
-                const T hyk = c ? hy.v[c - (c > 0)] : hy_km, hxk = c ? hx.v[c - (c > 0)] : hx_km;
-                // Same accumulation order as the reference kernels.
-                const T cx = ((hz.v[c] - hz_jm.v[c]) - hy.v[c]) + hyk;
-                const T cy = ((hx.v[c] - hxk) - hz.v[c]) + hz_im.v[c];
-                const T cz = ((hy.v[c] - hy_im.v[c]) - hx.v[c]) + hx_jm.v[c];
-                ex.v[c] = fma_(bc[0].v[c], cx, mul_(alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[0], c), ex.v[c]));
-                ey.v[c] = fma_(alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[0], c), ey.v[c], mul_(bc[1].v[c], cy));
-                ez.v[c] = fma_(alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[0], c), ez.v[c], mul_(bc[2].v[c], cz));
-                dxz[c] = hz.v[c] - hz_im.v[c];
-                dxy[c] = hy.v[c] - hy_im.v[c];
-                dyz[c] = hz.v[c] - hz_jm.v[c];
-                dyx[c] = hx.v[c] - hx_jm.v[c];
-                dzy[c] = hy.v[c] - hyk;
-                dzx[c] = hx.v[c] - hxk;
-            }
-            cell_psi<T, V, OV ? 0 : -1, true>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
-            if constexpr (OV)
-                cell_psi<T, V, 1, true>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, ex, ey, ez);
-            // lumped ports of one edge: the thread that owns the edge steps
-            // the element on the value it is about to store
-            for (int q = 0; q < d.n_lumped; ++q) {
-                const int4 at = d.lumped[q];
-                if (at.x != i || at.y != j || (unsigned)(at.z - k) >= (unsigned)V) continue;
-#pragma unroll
-                for (int c = 0; c < V; ++c) {
-                    if (at.z != k + c) continue;
-                    const T v = lumped_edge_step<T>(d.ports[q], d.pa, b,
-                                                    at.w == 0 ? ex.v[c] : (at.w == 1 ? ey.v[c] : ez.v[c]));
-                    if (at.w == 0) ex.v[c] = v;
-                    if (at.w == 1) ey.v[c] = v;
-                    if (at.w == 2) ez.v[c] = v;
-                }
-            }
-            if (k + V - 1 > g.nz) {
-                keep_pad(ex, k, g.nz);
-                keep_pad(ey, k, g.nz);
-                keep_pad(ez, k, g.nz);
-            }
-            stv<V>(E + o, ex);
-            stv<V>(E + vol + o, ey);
-            stv<V>(E + 2 * vol + o, ez);
-            hz_im = hz;
-            hy_im = hy;
-        }
+        for (int i = i0; i < i1; ++i, o += si)
+            cell_E<T, V, CK, UA, OV, ES>(p, d, p.e + fs, H, p.e_next + fs, b, i, j, k, o, zs, hz_im, hy_im);
     }
 }
 
@@ -317,51 +397,15 @@ __global__ void __launch_bounds__(kDirectThreads, direct_min_ctas<T, V>())
     bool zs;
     if (!direct_cell(d, g.ny, blockIdx.x * blockDim.x + threadIdx.x, V, j, k, zs)) return;
     const long long vol = g.vol;
-    const int si = (int)g.si, sj = (int)g.sj;
+    const int si = (int)g.si;
     const int i0 = blockIdx.y * d.np, i1 = min(i0 + d.np, g.nx + 1);
     for (int b = threadIdx.y; b < p.B; b += blockDim.y) {
-        T* H = p.h + (long long)b * 3 * vol;
-        const T* __restrict__ E = p.e + (long long)b * 3 * vol;
+        const long long fs = (long long)b * 3 * vol;
+        const T* E = p.e_next + fs;
         int o = (int)pidx(g, i1 - 1, j, k);
         Vec<T, V> ez_ip = ldv<V>(E + 2 * vol + o + si), ey_ip = ldv<V>(E + vol + o + si);
-        for (int i = i1 - 1; i >= i0; --i, o -= si) {
-            Vec<T, V> a[3], bc[3];
-            load_cell_coef<T, V, CK, UA>(p, 1, o, a, bc);
-            const Vec<T, V> ex = ldv<V>(E + o), ey = ldv<V>(E + vol + o), ez = ldv<V>(E + 2 * vol + o);
-            const Vec<T, V> ez_jp = ldv<V>(E + 2 * vol + o + sj), ex_jp = ldv<V>(E + o + sj);
-            const T ey_kp = E[vol + o + V], ex_kp = E[o + V];
-            Vec<T, V> hx = ldv<V>(H + o), hy = ldv<V>(H + vol + o), hz = ldv<V>(H + 2 * vol + o);
-            T dxz[V], dxy[V], dyz[V], dyx[V], dzy[V], dzx[V];
-#pragma unroll
-            for (int c = 0; c < V; ++c) {
-                const T eyk = c < V - 1 ? ey.v[(c + 1) % V] : ey_kp, exk = c < V - 1 ? ex.v[(c + 1) % V] : ex_kp;
-                const T cx = ((ez_jp.v[c] - ez.v[c]) - eyk) + ey.v[c];
-                const T cy = ((exk - ex.v[c]) - ez_ip.v[c]) + ez.v[c];
-                const T cz = ((ey_ip.v[c] - ey.v[c]) - ex_jp.v[c]) + ex.v[c];
-                hx.v[c] = fma_(alpha_of<T, V, UA>(a[0], bc[0].v[c], p.a0[1], c), hx.v[c], -mul_(bc[0].v[c], cx));
-                hy.v[c] = fma_(alpha_of<T, V, UA>(a[1], bc[1].v[c], p.a0[1], c), hy.v[c], -mul_(bc[1].v[c], cy));
-                hz.v[c] = fma_(alpha_of<T, V, UA>(a[2], bc[2].v[c], p.a0[1], c), hz.v[c], -mul_(bc[2].v[c], cz));
-                dxz[c] = ez_ip.v[c] - ez.v[c];
-                dxy[c] = ey_ip.v[c] - ey.v[c];
-                dyz[c] = ez_jp.v[c] - ez.v[c];
-                dyx[c] = ex_jp.v[c] - ex.v[c];
-                dzy[c] = eyk - ey.v[c];
-                dzx[c] = exk - ex.v[c];
-            }
-            cell_psi<T, V, OV ? 0 : -1, false>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
-            if constexpr (OV)
-                cell_psi<T, V, 1, false>(d, b, i, j, k, zs, bc, dxz, dxy, dyz, dyx, dzy, dzx, hx, hy, hz);
-            if (k + V - 1 > g.nz) {
-                keep_pad(hx, k, g.nz);
-                keep_pad(hy, k, g.nz);
-                keep_pad(hz, k, g.nz);
-            }
-            stv<V>(H + o, hx);
-            stv<V>(H + vol + o, hy);
-            stv<V>(H + 2 * vol + o, hz);
-            ez_ip = ez;
-            ey_ip = ey;
-        }
+        for (int i = i1 - 1; i >= i0; --i, o -= si)
+            cell_H<T, V, CK, UA, OV>(p, d, E, p.h + fs, p.h_next + fs, b, i, j, k, o, zs, ez_ip, ey_ip);
     }
 }
 
@@ -464,34 +508,38 @@ static DirectDiv direct_div(int n) {
 }
 
 // Grid of the direct kernels: V cells and np planes per thread, 128 threads,
-// the field sets of a cell in threadIdx.y (as many as there are warps).  which: 0 = E,
-// 1 = H.  Returns whether both faces of an axis reach one cell.
+// the field sets of a cell in threadIdx.y (as many as there are warps).
+// Returns whether both faces of an axis reach one cell.
 template <typename T>
-static bool direct_grid(const StencilArgs<T>& a, DirectArgs& d, int V, int which, dim3& grid, dim3& block) {
-    for (auto& x : d.ax) x = AxisSlabs{};
-    for (auto& x : d.ax) x.lo1 = 0x7fffffff;
-    for (int q = 0; q < a.nfaces; ++q) {
-        const FaceDev& f = a.f[q];
-        AxisSlabs& x = d.ax[f.axis];
-        const int hi = f.lo > 0 || x.n[0] > 0 ? 1 : 0;  // a face of the whole axis first, then the far side
-        if (hi) x.lo1 = f.lo;
-        x.n[hi] = f.n;
-        x.s0[hi] = f.dJ * f.pk;
-        x.s1[hi] = f.pk;
-        x.slab[hi] = (unsigned)f.slab;
-        x.set[hi] = 4 * f.slab;
-        x.psi[hi] = static_cast<T*>(f.psi) + 2 * which * f.slab;  // E1, E2 or H1, H2
-        x.bcc[hi] = f.bcc;
-        x.air[hi] = f.masked ? f.air + 2 * which * f.slab : nullptr;
-    }
+static bool direct_grid(const StencilArgs<T>& a, DirectArgs& d, int V, dim3& grid, dim3& block) {
     bool overlap = false;
-    for (const AxisSlabs& x : d.ax) overlap = overlap || x.n[0] > x.lo1;
+    for (int side = 0; side < 2; ++side) {
+        for (auto& x : d.ax[side]) x = AxisSlabs{};
+        for (auto& x : d.ax[side]) x.lo1 = 0x7fffffff;
+        for (int q = 0; q < a.nfaces; ++q) {
+            const FaceDev& f = a.f[q];
+            AxisSlabs& x = d.ax[side][f.axis];
+            const int hi = f.lo > 0 || x.n[0] > 0 ? 1 : 0;  // a face of the whole axis first, then the far side
+            if (hi) x.lo1 = f.lo;
+            x.n[hi] = f.n;
+            x.s0[hi] = f.dJ * f.pk;
+            x.s1[hi] = f.pk;
+            x.slab[hi] = (unsigned)f.slab;
+            x.set[hi] = 4 * f.slab;
+            x.psi[hi] = static_cast<T*>(f.psi) + 2 * side * f.slab;  // E1, E2 or H1, H2
+            x.psi_out[hi] = static_cast<T*>(d.ping_pong ? f.psi_next : f.psi) + 2 * side * f.slab;
+            x.bcc[hi] = f.bcc;
+            x.air[hi] = f.masked ? f.air + 2 * side * f.slab : nullptr;
+        }
+        for (const AxisSlabs& x : d.ax[side]) overlap = overlap || x.n[0] > x.lo1;
+    }
     const int nset = std::min(a.B, kDirectThreads / 32);
     block = dim3(kDirectThreads / nset / 32 * 32, nset, 1);
     if (d.np < 1) d.np = 1;
+    const AxisSlabs& z = d.ax[0][2];
     const int nvec = a.g.nz / V + 1;
-    d.n_low = std::min(nvec, (d.ax[2].n[0] + V - 1) / V);
-    const int high = d.ax[2].n[1] > 0 ? nvec - std::min(nvec, d.ax[2].lo1 / V) : 0;
+    d.n_low = std::min(nvec, (z.n[0] + V - 1) / V);
+    const int high = z.n[1] > 0 ? nvec - std::min(nvec, z.lo1 / V) : 0;
     d.n_mid = std::max(0, nvec - d.n_low - high);
     d.n_edge = nvec - d.n_mid;
     const long long rows = a.g.ny + 1;
@@ -503,10 +551,10 @@ static bool direct_grid(const StencilArgs<T>& a, DirectArgs& d, int V, int which
     return overlap;
 }
 
-template <typename T, int V, int CK>
+template <typename T, int V, int CK, bool ES>
 static void direct_launch(const StencilArgs<T>& a, DirectArgs d, int which, cudaStream_t s) {
     dim3 grid, block;
-    const bool overlap = direct_grid<T>(a, d, V, which, grid, block);
+    const bool overlap = direct_grid<T>(a, d, V, grid, block);
     // alpha read from memory: conductive or mixed coefficients, and small
     // meshes whose thick slabs overlap
     const auto go = [&](auto kE, auto kH) {
@@ -516,11 +564,11 @@ static void direct_launch(const StencilArgs<T>& a, DirectArgs d, int which, cuda
             kH<<<grid, block, 0, s>>>(a, d);
     };
     if (overlap)
-        go(k_update_E<T, V, CK, false, true>, k_update_H<T, V, CK, false, true>);
+        go(k_update_E<T, V, CK, false, true, ES>, k_update_H<T, V, CK, false, true>);
     else if (a.unit_alpha)
-        go(k_update_E<T, V, CK, true, false>, k_update_H<T, V, CK, true, false>);
+        go(k_update_E<T, V, CK, true, false, ES>, k_update_H<T, V, CK, true, false>);
     else
-        go(k_update_E<T, V, CK, false, false>, k_update_H<T, V, CK, false, false>);
+        go(k_update_E<T, V, CK, false, false, ES>, k_update_H<T, V, CK, false, false>);
 }
 
 // Meshes up to this many cells take one cell per thread: their step is the
@@ -532,19 +580,35 @@ static void direct_launch(const StencilArgs<T>& a, DirectArgs d, int which, cuda
 constexpr long long kScalarCells = 150000;
 
 template <typename T>
-void launch_direct_half(const StencilArgs<T>& a, const DirectArgs& d, int which, cudaStream_t s) {
+static bool direct_wide(const StencilArgs<T>& a) {
+    return (long long)(a.g.nx + 1) * (a.g.ny + 1) * (a.g.nz + 1) > kScalarCells;
+}
+
+template <typename T>
+void launch_direct_half(const StencilArgs<T>& a0, const DirectArgs& d, int which, cudaStream_t s) {
     constexpr int W = 16 / (int)sizeof(T);
-    const bool one = (long long)(a.g.nx + 1) * (a.g.ny + 1) * (a.g.nz + 1) <= kScalarCells;
-    const auto kind = [&](auto ck) {
+    StencilArgs<T> a = a0;
+    if (!d.ping_pong) {
+        a.e_next = a.e;
+        a.h_next = a.h;
+    }
+    const bool wide = direct_wide(a);
+    const auto kind = [&](auto ck, auto es) {
         constexpr int CK = decltype(ck)::value;
-        one ? direct_launch<T, 1, CK>(a, d, which, s) : direct_launch<T, W, CK>(a, d, which, s);
+        constexpr bool ES = decltype(es)::value;
+        wide ? direct_launch<T, W, CK, ES>(a, d, which, s) : direct_launch<T, 1, CK, ES>(a, d, which, s);
     };
-    if (a.coef_kind == kCoefF16)
-        kind(std::integral_constant<int, kCoefF16>());
+    using Native = std::integral_constant<int, kCoefNative>;
+    using F16 = std::integral_constant<int, kCoefF16>;
+    using BF16 = std::integral_constant<int, kCoefBF16>;
+    if (d.slab_bits)  // the slab step takes no bfloat16
+        a.coef_kind == kCoefF16 ? kind(F16(), std::true_type()) : kind(Native(), std::true_type());
+    else if (a.coef_kind == kCoefF16)
+        kind(F16(), std::false_type());
     else if (a.coef_kind == kCoefBF16)
-        kind(std::integral_constant<int, kCoefBF16>());
+        kind(BF16(), std::false_type());
     else
-        kind(std::integral_constant<int, kCoefNative>());
+        kind(Native(), std::false_type());
 }
 
 template <typename T>

@@ -50,7 +50,7 @@ def _problem(n, layers, alpha, batch, seed=3):
         prob.cpml.append(CpmlFace(face, b, c, ck, air))
     ey0 = nx * (ny + 1) * (nz + 1)
     for p in range(2):
-        i, j, k = nx // 2, ny // 2, (nz // 2 + p) % nz
+        i, j, k = nx // 2 + p, ny // 2, (nz // 2 + p) % nz  # an edge of its own also for one cell in z
         flat = ey0 + (i * ny + j) * (nz + 1) + k
         prob.lumped.append(LumpedPort(np.array([flat]), np.ones(1), np.array([dt / M_eps[flat]]), R=50.0,
                                       v_src=[rng.standard_normal(STEPS) for _ in range(batch)]))
@@ -165,3 +165,44 @@ def test_cpml_stays_fused_beside_clear_dispersion(n, layers, precision):
     for q, (a, b) in enumerate(zip(*out)):
         scale = float(np.max(np.abs(b)))
         assert scale > 0 and float(np.max(np.abs(a - b))) <= (TOL[precision] if q < 2 else 1e-5) * scale
+
+
+def _slab_case(name, precision):
+    from conftest import load_golden
+
+    from magnelio_b200.workloads import dispersive_slab
+
+    if name == "box":
+        return _problem((53, 53, 55), (6, 5, 4, 7, 5, 6), "pec", 1)
+    if name == "small_batch":
+        return _problem((20, 19, 31), (4, 4, 4, 4, 4, 4), "mixed", 2)
+    if name == "two_edge_port":  # stepped between the E and the H update: buffer to buffer
+        prob = _problem((53, 53, 55), (6, 6, 6, 6, 6, 6), "one", 1)
+        lp = prob.lumped[0]
+        lp.flat_idx = np.array([lp.flat_idx[0], lp.flat_idx[0] + 2 * (prob.nz + 1)])
+        lp.signs, lp.betas = np.ones(2), np.repeat(lp.betas, 2)
+        return prob
+    if name == "dispersive":
+        return dispersive_slab(26, 24, 45, seed=6, cpml_cells=4, n_freq=3)
+    return load_golden(name)[0]
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("name", ["box", "small_batch", "two_edge_port", "dispersive", "wg_dtbc", "planewave_box"])
+def test_slab_step_on_the_direct_kernels_matches_its_unit_lists(name, precision):
+    """Without a march depth the slab step runs on the direct kernels, in
+    place or from one buffer set to the other; with one it keeps its unit
+    lists.  Odd and even step counts, so both buffer sets end up current."""
+    out = []
+    for depth in (0, 9):
+        prob = _slab_case(name, precision)
+        with prob.build_engine(precision) as eng:
+            eng.configure_stencil("fused", 16, depth)
+            eng.step(20)
+            eng.step(STEPS - 20)
+            out.append([a for b in range(prob.batch) for a in (*eng.read_fields(b), *eng.read_vi(b))])
+    scale = [max(float(np.max(np.abs(a))) if a.size else 0.0 for a in out[1][q::4]) for q in range(4)]
+    for q, (a, b) in enumerate(zip(*out)):
+        assert np.all(np.isfinite(a))
+        if a.size:
+            assert float(np.max(np.abs(a - b))) <= (1 if q % 4 < 2 else 10) * TOL[precision] * scale[q % 4], q
