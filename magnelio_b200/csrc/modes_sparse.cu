@@ -22,6 +22,14 @@
 // rotates it onto the Ritz vectors; the residuals ||L x_j - theta_j x_j||
 // decide convergence.  Every loop is bounded; the routine reports the
 // iterations used and fails if the residuals do not reach the tolerance.
+//
+// A port plane's block (a few thousand rows, seven columns) is far too small
+// to fill the chip: the time is launches and host round trips.  So a filter
+// (up to 100 degrees) and the orthonormalisation of a block are one
+// cooperative launch each, their CTAs meeting at bounded grid barriers: on a
+// 104 x 46 plane with three modes the solve took 10.0 ms with a launch per
+// degree and some eight launches and two host reads per column, and 5.4 ms so
+// (7 iterations; 209 x 93: 15 ms).
 #include "fitb_common.cuh"
 
 #include <algorithm>
@@ -36,6 +44,37 @@ constexpr int kT = 256;
 
 int grid_for(long long work) {
     return (int)std::max<long long>(1, std::min<long long>((work + kT - 1) / kT, 148LL * 16));
+}
+
+__device__ double block_reduce(double x, double* sh) {
+    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
+    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
+    __syncthreads();
+    double r = 0.0;
+    if (threadIdx.x == 0)
+        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += sh[w];
+    return r;
+}
+
+// Barrier of all CTAs of a cooperative launch: `bar` counts arrivals (zeroed
+// before the launch), `round` is the caller's count of barriers so far.  The
+// wait is bounded; an expired one sets *err and every later barrier falls
+// through.
+constexpr unsigned kBarrierLimit = 1u << 24;
+__device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned& round, int* err) {
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const unsigned target = ++round * gridDim.x * gridDim.y;
+        __threadfence();
+        atomicAdd(bar, 1u);
+        unsigned v, tries = 0;
+        do {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
+        } while ((int)(v - target) < 0 && ++tries < kBarrierLimit && *(volatile int*)err == 0);
+        if ((int)(v - target) < 0) atomicExch(err, 1);
+        __threadfence();
+    }
+    __syncthreads();
 }
 
 // Yn = alpha (L Y) + beta Y + gamma X, blocks column-major (column j at j n)
@@ -54,14 +93,109 @@ __global__ void k_cheb(long long n, int k, const long long* rp, const long long*
     }
 }
 
-__device__ double block_reduce(double x, double* sh) {
-    for (int o = 16; o > 0; o >>= 1) x += __shfl_xor_sync(0xffffffffu, x, o);
-    if ((threadIdx.x & 31) == 0) sh[threadIdx.x >> 5] = x;
-    __syncthreads();
-    double r = 0.0;
-    if (threadIdx.x == 0)
-        for (int w = 0; w < (int)(blockDim.x >> 5); ++w) r += sh[w];
-    return r;
+// a reproducible start block: a hash of (row, column, seed) in [-1, 1)
+__device__ __forceinline__ double random_entry(long long r, long long c, unsigned seed) {
+    unsigned long long h = (unsigned long long)r * 0x9E3779B97F4A7C15ull ^
+                           ((unsigned long long)(c + 1) * 0xBF58476D1CE4E5B9ull) ^ ((unsigned long long)seed << 32);
+    h ^= h >> 31;
+    h *= 0x94D049BB133111EBull;
+    h ^= h >> 29;
+    return (double)(h >> 11) * (2.0 / 9007199254740992.0) - 1.0;
+}
+
+// The whole filter: degree d (from 1) of the recurrence with the factors
+// f[3 (d-1) ..], from P0 (the block) through P1, P2 in rotation; the last
+// degree's block is P[m % 3].  Other CTAs' rows change between degrees, so
+// they are read past the L1.
+struct ChebPlan {
+    double f[300];
+    double* P[3];
+    int m;
+};
+constexpr int kTF = 512;  // few CTAs, so that few meet at the barriers; column blockIdx.y
+__global__ void __launch_bounds__(kTF) k_filter(long long n, const long long* __restrict__ rp,
+                                               const long long* __restrict__ col, const double* __restrict__ val,
+                                               const __grid_constant__ ChebPlan p, unsigned* bar, int* err) {
+    unsigned round = 0;
+    const long long c0 = blockIdx.y * n;
+    for (int d = 1; d <= p.m; ++d) {
+        const double alpha = p.f[3 * d - 3], beta = p.f[3 * d - 2], gamma = p.f[3 * d - 1];
+        const double* y = p.P[(d - 1) % 3] + c0;
+        const double* x = p.P[(d + 1) % 3] + c0;  // the degree before y's
+        double* yn = p.P[d % 3] + c0;
+        for (long long i = blockIdx.x * (long long)kTF + threadIdx.x; i < n; i += (long long)gridDim.x * kTF) {
+            const double prev = d > 1 ? x[i] : 0.0;
+            double acc = 0.0;
+            for (long long q = rp[i]; q < rp[i + 1]; ++q) acc += val[q] * __ldcg(y + col[q]);
+            double r = alpha * acc + beta * __ldcg(y + i);
+            if (d > 1) r += gamma * prev;
+            yn[i] = r;
+        }
+        if (d < p.m) grid_barrier(bar, round, err);
+    }
+}
+
+// The columns of X orthonormal to the nz vectors Z and to one another:
+// classical Gram-Schmidt twice per column, a column that lost its rank
+// started afresh (up to four times, then *err = 2).  part: one row of partial
+// sums per CTA; they are added in CTA order, so the result does not depend on
+// timing.
+constexpr int kPart = 64;        // partial sums per CTA: nz + k + 1 of them used
+constexpr int kOrthoCtas = 128;  // CTAs at most
+__global__ void __launch_bounds__(kT) k_ortho(long long n, double* X, int k, const double* Z, int nz, double* part,
+                                              unsigned* bar, int* err) {
+    __shared__ double sh[32], coef[kPart];
+    unsigned round = 0, flip = 0;
+    const long long r0 = blockIdx.x * (long long)blockDim.x + threadIdx.x, stride = (long long)gridDim.x * blockDim.x;
+    // coef[q] = (q < nz ? Z_q : X_(q - nz)) . x for q < nc, and x . x at nc
+    // (two rows of partial sums in turn: one is written while a slower CTA
+    // still reads the other)
+    auto dots = [&](const double* x, int nc, bool cross) {
+        double* pt = part + (size_t)(flip ^= 1u) * kOrthoCtas * kPart;
+        for (int q = cross ? 0 : nc; q <= nc; ++q) {
+            const double* a = q == nc ? x : (q < nz ? Z + (long long)q * n : X + (long long)(q - nz) * n);
+            double s = 0.0;
+            for (long long r = r0; r < n; r += stride) s += a[r] * x[r];
+            s = block_reduce(s, sh);
+            if (threadIdx.x == 0) pt[blockIdx.x * kPart + q] = s;
+            __syncthreads();
+        }
+        grid_barrier(bar, round, err);
+        for (int q = (cross ? 0 : nc) + (int)threadIdx.x; q <= nc; q += blockDim.x) {
+            double s = 0.0;
+            for (unsigned c = 0; c < gridDim.x; ++c) s += __ldcg(pt + c * kPart + q);
+            coef[q] = s;
+        }
+        __syncthreads();
+    };
+    for (int c = 0; c < k; ++c) {
+        double* x = X + (long long)c * n;
+        const int nc = nz + c;
+        bool done = false;
+        for (int attempt = 0; attempt < 4 && !done; ++attempt) {
+            double before = 0.0;
+            for (int pass = 0; pass < 2; ++pass) {
+                dots(x, nc, true);
+                if (pass == 0) before = coef[nc];
+                for (long long r = r0; r < n; r += stride) {
+                    double s = 0.0;
+                    for (int q = 0; q < nc; ++q)
+                        s += coef[q] * (q < nz ? Z[(long long)q * n + r] : X[(long long)(q - nz) * n + r]);
+                    x[r] -= s;
+                }
+            }
+            dots(x, nc, false);
+            const double after = coef[nc];
+            done = after > 1e-20 * before && after > 0.0;
+            const double f = done ? 1.0 / sqrt(after) : 0.0;
+            for (long long r = r0; r < n; r += stride)
+                x[r] = done ? x[r] * f : random_entry(r, c, 7919u * (attempt + 1) + 13u);
+        }
+        if (!done) {
+            if (r0 == 0) atomicExch(err, 2);
+            return;  // every CTA: `after` is the same in all of them
+        }
+    }
 }
 
 // out[i * nb + j] = A_i . B_j for i < na, j < nb (one block per pair)
@@ -76,23 +210,6 @@ __global__ void __launch_bounds__(kT) k_gram(long long n, const double* A, int n
     for (long long r = threadIdx.x; r < n; r += blockDim.x) s += a[r] * b[r];
     s = block_reduce(s, sh);
     if (threadIdx.x == 0) out[i * nb + j] = s;
-}
-
-// x_c -= sum_i coef[i * ld + c] A_i for the columns c < nc of X (A has na columns)
-__global__ void k_subtract(long long n, double* X, int nc, const double* A, int na, const double* coef, int ld) {
-    const long long total = n * nc;
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
-         t += (long long)gridDim.x * blockDim.x) {
-        const long long c = t / n, r = t - c * n;
-        double s = 0.0;
-        for (int i = 0; i < na; ++i) s += coef[i * ld + c] * A[(long long)i * n + r];
-        X[t] -= s;
-    }
-}
-
-__global__ void k_scale(long long n, double* x, double f) {
-    for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x)
-        x[t] *= f;
 }
 
 // Out_j = sum_i In_i R[i * k + j]
@@ -122,18 +239,12 @@ __global__ void __launch_bounds__(kT) k_residual(long long n, const double* W, c
     if (threadIdx.x == 0) out[j] = s;
 }
 
-// a reproducible start block: a hash of (row, column, seed) in [-1, 1)
 __global__ void k_random(long long n, int c0, int nc, unsigned seed, double* X) {
     const long long total = n * nc;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < total;
          t += (long long)gridDim.x * blockDim.x) {
         const long long c = t / n + c0, r = t - (t / n) * n;
-        unsigned long long h = (unsigned long long)r * 0x9E3779B97F4A7C15ull ^
-                               ((unsigned long long)(c + 1) * 0xBF58476D1CE4E5B9ull) ^ ((unsigned long long)seed << 32);
-        h ^= h >> 31;
-        h *= 0x94D049BB133111EBull;
-        h ^= h >> 29;
-        X[c * n + r] = (double)(h >> 11) * (2.0 / 9007199254740992.0) - 1.0;
+        X[c * n + r] = random_entry(r, c, seed);
     }
 }
 
@@ -194,58 +305,61 @@ int sparse_lowest_eigs(long long n, const long long* rp, const long long* col, c
     const int k = (int)std::min<long long>(n_modes + std::max(4, n_modes), n - n_null);
     if (k < n_modes || !(b > 0.0)) return -1;
     const size_t blk = (size_t)n * k;
+    // five allocations of a few hundred KB rather than one: the driver serves
+    // those from chunks it holds, while one of more than a MB is mapped and
+    // unmapped on every call (measured: 5.4 ms a solve against 8.6)
     double *X = nullptr, *Y = nullptr, *Yn = nullptr, *W = nullptr, *sm = nullptr;
     auto release = [&]() { cudaFree(X), cudaFree(Y), cudaFree(Yn), cudaFree(W), cudaFree(sm); };
     if (cudaMalloc(&X, blk * 8) || cudaMalloc(&Y, blk * 8) || cudaMalloc(&Yn, blk * 8) || cudaMalloc(&W, blk * 8) ||
-        cudaMalloc(&sm, 4096 * 8)) {
+        cudaMalloc(&sm, (4096 + 2 * (size_t)kOrthoCtas * kPart) * 8)) {
         release();
         return -2;
     }
-    double* coef = sm;          // up to 64 coefficients
     double* H = sm + 64;        // k x k
     double* R = sm + 64 + 1024; // k x k
     double* th = sm + 64 + 2048;
     double* rs = sm + 64 + 2048 + 64;
-    const int g_blk = grid_for((long long)blk), g_n = grid_for(n);
+    const int g_blk = grid_for((long long)blk);
     auto host_read = [&](const double* d, double* h, int cnt) {
         cudaMemcpyAsync(h, d, cnt * sizeof(double), cudaMemcpyDeviceToHost, s);
         return cudaStreamSynchronize(s) == cudaSuccess;
     };
-    // column c of X orthonormal to the null vectors and to columns < c
-    auto ortho_column = [&](int c) -> int {
-        double* xc = X + (size_t)c * n;
-        double before = 0.0, after = 0.0;
-        for (int attempt = 0; attempt < 4; ++attempt) {
-            k_gram<<<1, kT, 0, s>>>(n, xc, 1, xc, 1, coef);
-            if (!host_read(coef, &before, 1)) return -2;
-            for (int pass = 0; pass < 2; ++pass) {
-                if (n_null) {
-                    k_gram<<<n_null, kT, 0, s>>>(n, Z, n_null, xc, 1, coef);
-                    k_subtract<<<g_n, kT, 0, s>>>(n, xc, 1, Z, n_null, coef, 1);
-                }
-                if (c) {
-                    k_gram<<<c, kT, 0, s>>>(n, X, c, xc, 1, coef);
-                    k_subtract<<<g_n, kT, 0, s>>>(n, xc, 1, X, c, coef, 1);
-                }
-            }
-            k_gram<<<1, kT, 0, s>>>(n, xc, 1, xc, 1, coef);
-            if (!host_read(coef, &after, 1)) return -2;
-            if (after > 1e-20 * before && after > 0.0) {
-                k_scale<<<g_n, kT, 0, s>>>(n, xc, 1.0 / std::sqrt(after));
-                return 0;
-            }
-            // the column lost its rank: start it afresh
-            k_random<<<g_n, kT, 0, s>>>(n, c, 1, 7919u * (attempt + 1) + 13u, X);
-        }
-        return -5;
+    // cooperative launches: as many CTAs as the rows need and the chip holds
+    int dev = 0, sms = 148, occ_f = 1;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ_f, k_filter, kTF, 0);
+    const dim3 g_f((unsigned)std::max<long long>(1, std::min<long long>((n + kTF - 1) / kTF, (long long)sms * occ_f / k)),
+                   (unsigned)k);
+    const int g_o = (int)std::max<long long>(1, std::min<long long>((n + kT - 1) / kT, std::min(sms, kOrthoCtas)));
+    unsigned* bar = reinterpret_cast<unsigned*>(sm + 64 + 2048 + 256);
+    int* err = reinterpret_cast<int*>(bar + 1);
+    double* part = sm + 4096;
+    auto coop = [&](const void* f, dim3 grid, int threads, void** args) {
+        if (cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), s) != cudaSuccess) return -2;
+        return cudaLaunchCooperativeKernel(f, grid, dim3(threads), args, 0, s) == cudaSuccess ? 0 : -2;
     };
+    // every column of X orthonormal to the null vectors and to the ones before
+    // it; the outcome is read with the next host read
+    auto ortho = [&]() -> int {
+        long long nn = n;
+        int kk = k, nz = n_null;
+        const double* z = Z;
+        double* x = X;
+        void* args[] = {&nn, &x, &kk, &z, &nz, &part, &bar, &err};
+        return coop((const void*)k_ortho, dim3(g_o), kT, args);
+    };
+    auto outcome = [&](int e) { return e == 2 ? -5 : (e ? -2 : 0); };
     std::vector<double> hH((size_t)k * k), w, V, hres(k);
     double a = 0.0, a0 = 0.0, best = 1e300;
     int since_best = 0, it = 0, rc = -4;
     auto rayleigh_ritz = [&]() -> int {
         k_cheb<<<g_blk, kT, 0, s>>>(n, k, rp, col, val, X, X, W, 1.0, 0.0, 0.0);
         k_gram<<<k * k, kT, 0, s>>>(n, X, k, W, k, H);
+        int e = 0;
+        cudaMemcpyAsync(&e, err, sizeof(int), cudaMemcpyDeviceToHost, s);
         if (!host_read(H, hH.data(), k * k)) return -2;
+        if (e) return outcome(e);
         for (int i = 0; i < k; ++i)
             for (int j = i + 1; j < k; ++j) hH[i * k + j] = hH[j * k + i] = 0.5 * (hH[i * k + j] + hH[j * k + i]);
         jacobi_eigen(k, hH, w, V);
@@ -260,14 +374,11 @@ int sparse_lowest_eigs(long long n, const long long* rp, const long long* col, c
         return 0;
     };
     k_random<<<g_blk, kT, 0, s>>>(n, 0, k, 1u, X);
-    for (int c = 0; c < k; ++c)
-        if (int e = ortho_column(c)) {
-            release();
-            return e;
-        }
-    if (int e = rayleigh_ritz()) {
+    int e0 = ortho();
+    if (e0 == 0) e0 = rayleigh_ritz();
+    if (e0) {
         release();
-        return e;
+        return e0;
     }
     const int degree = 100, max_iter = 400;
     for (it = 1; it <= max_iter; ++it) {
@@ -283,21 +394,34 @@ int sparse_lowest_eigs(long long n, const long long* rp, const long long* col, c
         // higher gain would fold the whole block onto one vector)
         const double x0 = (a + b - 2.0 * a0) / (b - a);
         const int m = (int)std::min<double>(degree, std::max(1.0, 19.0 / std::acosh(std::max(x0, 1.0 + 1e-12))));
-        k_cheb<<<g_blk, kT, 0, s>>>(n, k, rp, col, val, X, X, Y, sigma / e, -c * sigma / e, 0.0);
+        ChebPlan plan;
+        plan.m = m;
+        plan.P[0] = X;
+        plan.P[1] = Y;
+        plan.P[2] = Yn;
+        plan.f[0] = sigma / e;
+        plan.f[1] = -c * sigma / e;
+        plan.f[2] = 0.0;
         for (int d = 2; d <= m; ++d) {
             const double s2 = 1.0 / (tau - sigma);
-            k_cheb<<<g_blk, kT, 0, s>>>(n, k, rp, col, val, Y, X, Yn, 2.0 * s2 / e, -2.0 * s2 * c / e, -sigma * s2);
-            std::swap(X, Y);   // X <- Y (previous), Y <- Yn (current)
-            std::swap(Y, Yn);
+            plan.f[3 * d - 3] = 2.0 * s2 / e;
+            plan.f[3 * d - 2] = -2.0 * s2 * c / e;
+            plan.f[3 * d - 1] = -sigma * s2;
             sigma = s2;
         }
-        std::swap(X, Y);       // the filtered block
-        for (int cc = 0; cc < k; ++cc)
-            if (int er = ortho_column(cc)) {
-                release();
-                return er;
-            }
-        if (int er = rayleigh_ritz()) {
+        long long nn = n;
+        void* args[] = {&nn, &rp, &col, &val, &plan, &bar, &err};
+        int er = coop((const void*)k_filter, g_f, kTF, args);
+        // the filtered block to X
+        X = plan.P[m % 3];
+        Y = plan.P[(m + 1) % 3];
+        Yn = plan.P[(m + 2) % 3];
+        int ferr = 0;
+        if (er == 0 && cudaMemcpyAsync(&ferr, err, sizeof(int), cudaMemcpyDeviceToHost, s) != cudaSuccess) er = -2;
+        if (er == 0) er = ortho();
+        if (er == 0) er = rayleigh_ritz();
+        if (er == 0) er = outcome(ferr);
+        if (er) {
             release();
             return er;
         }
