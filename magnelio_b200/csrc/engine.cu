@@ -267,6 +267,7 @@ struct Handle {
     DevBuf d_band;
     DevBuf d_lumped, d_modal, d_dft;
     int dft_blocks = 0;
+    DftPack dft_pack{};
     size_t dft_smem = 0;
     DevBuf ticket;  // CTA completion counter of the monitor launch
     int launches_per_step = 0;
@@ -693,6 +694,7 @@ void refresh_port_tables(Handle& H) {
         dd.push_back(d);
     }
     upload(H.d_dft, dd);
+    for (size_t q = 0; q < dd.size() && q < (size_t)kDftPack; ++q) H.dft_pack.d[q] = dd[q];
     if (H.stencil_mode == kModeFused) build_fix_cells(H);
     if (H.stencil_mode == kModeFused && is_slab_variant(H.fused_variant)) build_slab_units(H);
     H.dft_blocks = sb;
@@ -1210,7 +1212,7 @@ int enqueue_step_fused(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_step<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.d_dft.as<DftDev>(),
+        launch_dft_step<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.dft_pack, H.d_dft.as<DftDev>(),
                            (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), 0,
                            H.ticket.as<unsigned>(), H.stream);
         ++n;
@@ -1272,7 +1274,7 @@ int enqueue_step(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.d_dft.as<DftDev>(),
+        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.dft_pack, H.d_dft.as<DftDev>(),
                            (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), advance ? 1 : 0,
                            H.ticket.as<unsigned>(), H.stream);
         ++n;

@@ -491,9 +491,13 @@ int dft_blocks(long long work);
 // ones (dynamic shared memory for the largest monitor's phasors).  done = 1:
 // the step counter is already advanced; 0: this launch advances it (its last
 // CTA, through `ticket`).
+constexpr int kDftPack = 8;
+struct DftPack {
+    DftDev d[kDftPack];  // the first monitors, as in the device table `devs`
+};
 template <typename T>
 void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                     const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
+                     const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
                      unsigned* ticket, cudaStream_t s);
 // Host-requested flush of the first kc slots of one monitor.
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s);

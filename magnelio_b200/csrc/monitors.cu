@@ -114,18 +114,34 @@ __device__ __forceinline__ void flush_cell(const DftDev& d, int kc, int tsel, co
 // an earlier kernel of the step has advanced it; otherwise the last CTA of
 // this launch does, through `ticket`.  Staging and flushing were two launches
 // before, the second one empty on K - 1 of K steps: on a 97 x 104 x 89 mesh
-// with three planes of 16 frequencies the two cost 13 us per step.
-template <typename T>
+// with three planes of 16 frequencies the two cost 13 us per step.  The
+// launch is short, so its chain counts: up to kDftPack descriptors travel as
+// kernel arguments (else a block's first loads are a descriptor from HBM or
+// L2, one after the other per monitor), and the slot arithmetic is 32-bit
+// while the step count is.
+template <typename T, bool PACK>
 __global__ void __launch_bounds__(kThreads, 3)
     k_dft_step(const T* __restrict__ e, const T* __restrict__ h, long long e_block, long long h_block, Geom g, int B,
-               const DftDev* __restrict__ devs, int nmon, long long* step, int done, unsigned* ticket) {
+               const __grid_constant__ DftPack pack, const DftDev* __restrict__ devs_dev, int nmon, long long* step,
+               int done, unsigned* ticket) {
     extern __shared__ float2 sw[];
+    const DftDev* devs = PACK ? pack.d : devs_dev;
     const DftDev& d = devs[monitor_of_block(devs, nmon)];
     const int lb = blockIdx.x - d.sblk0;
     const long long n = *step - done;
-    if (n % d.stride == 0) {
-        const long long cnt = recorded_upto(n, d.stride) - recorded_upto(*d.base - 1, d.stride);
-        const int slot = (int)((cnt - 1) % d.K);
+    const long long base = *d.base;
+    const bool narrow = n < 0x7fffffffLL;
+    if (narrow ? (unsigned)n % (unsigned)d.stride == 0 : n % d.stride == 0) {
+        // recorded steps from base to n, less one, within the block of K
+        int slot;
+        if (narrow) {
+            const unsigned st = (unsigned)d.stride;
+            const unsigned before = base > 0 ? (unsigned)(base - 1) / st + 1u : 0u;
+            slot = (int)(((unsigned)n / st - before) % (unsigned)d.K);
+        } else {
+            const long long cnt = recorded_upto(n, d.stride) - recorded_upto(base - 1, d.stride);
+            slot = (int)((cnt - 1) % d.K);
+        }
         const bool flush = slot == d.K - 1;
         // this step's phasors: for the later steps of the block, and (every
         // CTA for itself) for the flush
@@ -212,9 +228,14 @@ int dft_blocks(long long work) {
 
 template <typename T>
 void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                     const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
-                     unsigned* ticket, cudaStream_t s) {
-    k_dft_step<T><<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, devs, nmon, step, done, ticket);
+                     const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step,
+                     int done, unsigned* ticket, cudaStream_t s) {
+    if (nmon <= kDftPack)
+        k_dft_step<T, true>
+            <<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, pack, devs, nmon, step, done, ticket);
+    else
+        k_dft_step<T, false>
+            <<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, pack, devs, nmon, step, done, ticket);
 }
 
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s) {
@@ -223,8 +244,10 @@ void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s) {
 }
 
 template void launch_dft_step<float>(const float*, const float*, long long, long long, const Geom&, int,
-                                     const DftDev*, int, int, size_t, long long*, int, unsigned*, cudaStream_t);
+                                     const DftPack&, const DftDev*, int, int, size_t, long long*, int, unsigned*,
+                                     cudaStream_t);
 template void launch_dft_step<double>(const double*, const double*, long long, long long, const Geom&, int,
-                                      const DftDev*, int, int, size_t, long long*, int, unsigned*, cudaStream_t);
+                                      const DftPack&, const DftDev*, int, int, size_t, long long*, int, unsigned*,
+                                      cudaStream_t);
 
 }  // namespace fitb

@@ -206,3 +206,31 @@ def test_slab_step_on_the_direct_kernels_matches_its_unit_lists(name, precision)
         assert np.all(np.isfinite(a))
         if a.size:
             assert float(np.max(np.abs(a - b))) <= (1 if q % 4 < 2 else 10) * TOL[precision] * scale[q % 4], q
+
+
+@pytest.mark.parametrize("count", [1, 8, 9])
+def test_monitor_slots_with_and_without_packed_descriptors(count):
+    """Monitors of strides 1 .. count, up to and past the number whose
+    descriptors travel as kernel arguments: the bins are the DFT sums of the
+    fields read after every step, over whole and partial slot blocks."""
+    from magnelio_b200.problem import DftMonitor
+
+    prob = _problem((9, 8, 11), (0,) * 6, "one", 1)
+    freqs = np.array([1e9, 7e9])
+    prob.monitors = [DftMonitor(((1, 7), (2, 8), (3, 9)), ("Ez",), freqs, stride) for stride in range(1, count + 1)]
+    want = [np.zeros((2, 6, 6, 6), complex) for _ in range(count)]
+    steps = 70
+    with prob.build_engine("double") as eng:
+        shape = eng.shapes["Ez"]
+        for n in range(steps):
+            eng.step(1)
+            ez = eng.read_fields()[0][-int(np.prod(shape)):].reshape(shape)
+            a = ez[1:8, 2:9, 3:9]
+            cell = 0.25 * (a[:-1, :-1] + a[1:, :-1] + a[:-1, 1:] + a[1:, 1:]) / prob.dz[None, None, 3:9]
+            for m in range(count):
+                if n % (m + 1) == 0:
+                    w = np.exp(2j * np.pi * freqs * n * prob.dt) * (m + 1) * prob.dt
+                    want[m] += w[:, None, None, None] * cell
+        for m in range(count):
+            got = eng.read_dft(m, "Ez")
+            assert np.max(np.abs(got - want[m])) <= 1e-5 * np.max(np.abs(want[m]))  # float32 samples and bins
