@@ -733,12 +733,17 @@ def run_b200(args, world, rank, local):
     peak, peak_kind = _peaks()
     tile = stencil_cfg["kind"] == "fused" and TILE_VARIANT_BASE <= stencil_cfg["variant"] < SLAB_VARIANT_BASE
     slab = stencil_cfg["kind"] == "fused" and stencil_cfg["variant"] >= SLAB_VARIANT_BASE
-    if slab:
+    # the slab step without a given march depth runs on the direct kernels
+    lists = slab and tuned is not None and tuned.ichunk > 0
+    if lists:
         kernel = "k_step_slab (one stencil step, CPML inside the march)"
         traffic = _traffic("slab_step", n, cpml_cells) if B == 1 else None
     elif tile:
         kernel = "k_step_tile + CPML passes (one stencil step)"
         traffic = _traffic("tile_step", n, cpml_cells) if B == 1 else None
+    elif slab or stencil_cfg["kind"] == "simple":
+        kernel = "k_update_E + k_update_H (one stencil step on the direct kernels)"
+        traffic = _traffic("direct", n, cpml_cells) if B == 1 else None
     else:
         kernel = "update_E + update_H (one stencil step)"
         traffic = _traffic("update_E+update_H", n) if stencil_cfg["kind"] == "stream" and B == 1 else None

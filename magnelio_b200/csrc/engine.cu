@@ -1274,8 +1274,8 @@ int enqueue_step(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.dft_pack, H.d_dft.as<DftDev>(),
-                           (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), advance ? 1 : 0,
+        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.dft_pack,
+                           H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), advance ? 1 : 0,
                            H.ticket.as<unsigned>(), H.stream);
         ++n;
     } else if (!advance) {
