@@ -63,8 +63,10 @@ struct HostLanes {
         const size_t pieces = (bytes + kPiece - 1) / kPiece;
         const unsigned hw = std::max(1u, std::thread::hardware_concurrency());
         const int lanes = (int)std::min<size_t>({(size_t)kLanes, (size_t)hw, std::max<size_t>(1, pieces)});
-        const cudaError_t rc = prepare(lanes);
-        if (rc != cudaSuccess) return rc;
+        if (prepare(lanes) != cudaSuccess) {
+            cudaGetLastError();
+            return read_pageable(src, bytes, s, sink);
+        }
         std::atomic<size_t> next{0};
         std::atomic<int> err{0};
         const auto work = [&](int lane) {
@@ -82,6 +84,7 @@ struct HostLanes {
             if (e != cudaSuccess) err.store((int)e);
         };
         std::vector<std::thread> pool;
+        pool.reserve(lanes);
         try {
             for (int t = 1; t < lanes; ++t) pool.emplace_back(work, t);
         } catch (const std::system_error&) {
@@ -90,6 +93,19 @@ struct HostLanes {
         work(0);
         for (auto& t : pool) t.join();
         return (cudaError_t)err.load();
+    }
+
+    // Where no page-locked memory is to be had: one thread, a pageable piece.
+    static cudaError_t read_pageable(const void* src, size_t bytes, cudaStream_t s, const Sink& sink) {
+        std::vector<char> piece(std::min(kPiece, bytes));
+        cudaError_t e = cudaSuccess;
+        for (size_t off = 0; off < bytes && e == cudaSuccess; off += kPiece) {
+            const size_t n = std::min(kPiece, bytes - off);
+            e = cudaMemcpyAsync(piece.data(), static_cast<const char*>(src) + off, n, cudaMemcpyDeviceToHost, s);
+            if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+            if (e == cudaSuccess) sink(off, piece.data(), n);
+        }
+        return e;
     }
 };
 
