@@ -496,6 +496,16 @@ void invalidate_graphs(Handle& H) {
     H.graphs_valid = false;
 }
 
+// Some part of the problem was added, replaced or moved in memory: the tables,
+// the plans derived from them (which ports step inside the E kernel, where the
+// CPML may stay fused, the H cells beside written edges, the slab step's units)
+// and the graphs are made again before the next step.  Every call that changes
+// a part ends here, whichever plans read it.
+void problem_changed(Handle& H) {
+    H.port_tables_dirty = true;
+    invalidate_graphs(H);
+}
+
 // Recorder and DTBC history capacity (steps).  Growth keeps the contents
 // and invalidates the captured graphs (they hold the old pointers).
 void ensure_capacity(Handle& H, long long need) {
@@ -546,8 +556,7 @@ void ensure_capacity(Handle& H, long long need) {
     }
     legacy_sync("capacity copy sync");
     H.cap = ncap;
-    H.port_tables_dirty = true;
-    invalidate_graphs(H);
+    problem_changed(H);
 }
 
 // H cells whose update reads an E edge that a port writes between the E and
@@ -1506,8 +1515,7 @@ void set_form(Handle& H, int kind, int variant, int ichunk) {
         H.splan.ichunk = c;
         H.splan.grid_z = (nplanes + c - 1) / c;
     }
-    H.port_tables_dirty = true;
-    invalidate_graphs(H);
+    problem_changed(H);
 }
 
 template <typename T>
@@ -1957,8 +1965,7 @@ int fitb_set_coeffs(fitb_handle* h, const double* alpha_e, const double* beta_e,
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
     fitb::find_unit_alpha(H);
-    H.port_tables_dirty = true;  // the slab step's dead-unit plan reads the coefficients
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2012,8 +2019,7 @@ int fitb_build_materials(fitb_handle* h, const double* dx, const double* dy, con
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
     fitb::find_unit_alpha(H);
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2067,8 +2073,7 @@ int fitb_set_coeffs_native(fitb_handle* h, const void* alpha_e, const void* beta
     H.coeffs_set = true;
     fitb::compact_coeffs(H);
     fitb::find_unit_alpha(H);
-    H.port_tables_dirty = true;  // the slab step's dead-unit plan reads the coefficients
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2090,7 +2095,7 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind) {
     fitb::plan_stencil(H);
     fitb::compact_coeffs(H);
     fitb::find_unit_alpha(H);
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2208,8 +2213,7 @@ int fitb_add_cpml(fitb_handle* h, int32_t face, int32_t n_pml, const double* b, 
         fitb::add_cpml_impl<float>(H, face, n_pml, b, c, ck_, air);
     else
         fitb::add_cpml_impl<double>(H, face, n_pml, b, c, ck_, air);
-    H.port_tables_dirty = true;  // plans that depend on the slabs
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2254,8 +2258,7 @@ int fitb_add_lumped(fitb_handle* h, int32_t n_edges, const int64_t* flat_e_idx, 
     H.cap = 0;
     H.recV.release();
     H.recI.release();
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2276,8 +2279,7 @@ int fitb_set_lumped_source(fitb_handle* h, int32_t id, int32_t b, int64_t n_samp
     fitb::upload(lp.src, tab);
     lp.dev.src = lp.src.as<double>();
     lp.dev.n_src = n_new;
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2425,8 +2427,7 @@ int fitb_add_modal_port(fitb_handle* h, const fitb_modal_desc* d, int32_t* out_i
         other->shist.release();
     }
     fitb::ensure_capacity(H, want);
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2446,8 +2447,7 @@ int fitb_set_dtbc_kernel(fitb_handle* h, int32_t port, int32_t mode, int32_t n_k
     fitb::upload(mp.ktab[mode], tab);
     mp.dev.ktab[mode] = mp.ktab[mode].as<double>();
     mp.dev.n_tables = *std::max_element(mp.n_tables_mode.begin(), mp.n_tables_mode.end());
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2490,8 +2490,7 @@ int fitb_build_dtbc_kernel(fitb_handle* h, int32_t port, int32_t mode, int64_t n
     fitb::upload(mp.ktab[mode], mp.ktabs[(size_t)mode]);
     mp.dev.ktab[mode] = mp.ktab[mode].as<double>();
     mp.dev.n_tables = *std::max_element(mp.n_tables_mode.begin(), mp.n_tables_mode.end());
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2524,8 +2523,7 @@ int fitb_set_modal_source(fitb_handle* h, int32_t port, int32_t b, int32_t mode,
     fitb::upload(mp.buflen, mp.buflen_host);
     mp.dev.exc_mode = mp.exc.as<int>();
     mp.dev.buf_len = mp.buflen.as<int>();
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2619,7 +2617,7 @@ int fitb_add_dispersion_block(fitb_handle* h, int32_t side, int64_t n_states, co
     dv.uoff = D.d_uoff.as<long long>();
     dv.ustart = D.d_ustart.as<int>();
     dv.ustate = D.d_ustate.as<long long>();
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2711,8 +2709,7 @@ int fitb_add_band_port(fitb_handle* h, const fitb_band_desc* d, int32_t* out_id)
     // the recorder and the histories are sized for the new channel count
     H.cap = 0;
     fitb::ensure_capacity(H, 1);
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2729,8 +2726,7 @@ int fitb_set_band_kernel(fitb_handle* h, int32_t port, int32_t incoming, int32_t
     tab.insert(tab.end(), L, L + (size_t)n_kernel * bp.p * bp.p);
     nt += 1;
     fitb::upload(incoming ? bp.kin : bp.kout, tab);
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2755,8 +2751,7 @@ int fitb_set_band_source(fitb_handle* h, int32_t port, int32_t b, int64_t n_samp
     bp.src_on_host[(size_t)b] = 1;
     fitb::upload(bp.src, tab);
     fitb::upload(bp.src_on, bp.src_on_host);
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2836,7 +2831,7 @@ int fitb_add_sibc_block(fitb_handle* h, int64_t n_faces, const int64_t* idx, con
     dv.uoff = S.d_uoff.as<long long>();
     dv.ustart = S.d_ustart.as<int>();
     dv.ustate = S.d_ustate.as<long long>();
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -2905,8 +2900,7 @@ int fitb_add_plane_wave(fitb_handle* h, const fitb_plane_wave_desc* d, int32_t* 
     fitb::upload(pw->scale, pw->scale_host);
     dv.scale = pw->scale.as<double>();
     H.pws.push_back(std::move(pw));
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     if (out_id) *out_id = (int32_t)H.pws.size() - 1;
     FITB_CATCH
 }
@@ -2988,8 +2982,7 @@ int fitb_add_dft_monitor(fitb_handle* h, const fitb_dft_desc* d, int32_t* out_id
     m->i0 = d->i0; m->i1 = d->i1; m->j0 = d->j0; m->j1 = d->j1; m->k0 = d->k0; m->k1 = d->k1;
     if (out_id) *out_id = (int32_t)H.dft.size();
     H.dft.push_back(std::move(m));
-    H.port_tables_dirty = true;
-    fitb::invalidate_graphs(H);
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 
@@ -3081,10 +3074,10 @@ int fitb_time_stencil(fitb_handle* h, int32_t n_iter, double* ms_e, double* ms_h
     if (n_iter < 1 || !ms_e || !ms_h) fail(FITB_ERR_ARG, "bad argument");
     cudaEvent_t ev[3];
     for (auto& x : ev) ck(cudaEventCreate(&x), "event");
+    fitb::refresh_port_tables(H);  // the plans the launches follow
     if (H.stencil_mode == fitb::kModeFused) {
         // the whole E + H pass, alternating buffer sets; an even count
         // leaves the current set where it was
-        fitb::refresh_port_tables(H);  // the slab form's unit lists
         const int n2 = 2 * ((n_iter + 1) / 2);
         ck(cudaEventRecord(ev[0], H.stream), "event record");
         int nl = 0;
@@ -3406,8 +3399,7 @@ int fitb_state_import(fitb_handle* h, const void* buf, size_t len) {
     else
         fitb::read_state<double>(H, r);
     if (r.left != 0) fail(FITB_ERR_ARG, "state buffer has %zu trailing bytes", r.left);
-    fitb::invalidate_graphs(H);
-    H.port_tables_dirty = true;
+    fitb::problem_changed(H);
     FITB_CATCH
 }
 

@@ -234,3 +234,54 @@ def test_monitor_slots_with_and_without_packed_descriptors(count):
         for m in range(count):
             got = eng.read_dft(m, "Ez")
             assert np.max(np.abs(got - want[m])) <= 1e-5 * np.max(np.abs(want[m]))  # float32 samples and bins
+
+
+def _late_dispersion(prob, where):
+    """A one-pole block on E entries inside the xmin slab, or on and beside
+    the first port's edge (clear of every slab); coupling 5 % of a field step."""
+    from magnelio_b200.problem import Dispersion, DispersionBlock
+
+    if where == "slab":
+        idx = np.flatnonzero(prob.beta_E[:2 * (prob.ny + 1) * (prob.nz + 1)])
+    else:
+        idx = prob.lumped[0].flat_idx[0] + np.arange(-2, 3)
+        idx = idx[prob.beta_E[idx] != 0]
+    block = DispersionBlock(idx.astype(np.int64), 0.05 / prob.beta_E[idx], np.zeros(1, np.int32), np.array([0.9]),
+                            np.array([1.0]), np.ones(1))
+    return [Dispersion("E", [block])]
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("form", [None, ("fused", 16), ("stream",)])
+@pytest.mark.parametrize("where", ["slab", "port"])
+def test_dispersion_added_to_a_prepared_handle(where, form, precision):
+    """A block added after the handle prepared its step (a step of zero) is
+    taken as if it had been there before: the CPML of a slab that it reaches
+    into follows the pole update, a port on its edge follows it too, and the
+    slab step recomputes H beside it (or refuses the block in a slab)."""
+    from magnelio_b200._lib import FitbError
+
+    prob = _problem((26, 24, 45), (4,) * 6, "one", 1)
+    disp = _late_dispersion(prob, where)
+    out = []
+    for late in (True, False):
+        prob.dispersion = [] if late else disp
+        with prob.build_engine(precision) as eng:
+            if form and late:
+                eng.configure_stencil(*form)
+            if late:
+                eng.reserve_steps(STEPS)
+                eng.step(0)
+                for side in disp:
+                    for block in side.blocks:
+                        eng.add_dispersion_block(side.side, block)
+            if form == ("fused", 16) and where == "slab":
+                with pytest.raises(FitbError, match="outside the CPML slabs"):
+                    eng.step(STEPS) if late else eng.configure_stencil(*form)
+                continue
+            if form and not late:
+                eng.configure_stencil(*form)
+            eng.step(STEPS)
+            out.append((*eng.read_fields(), *eng.read_vi(), eng.read_dft(0, "Ex")))
+    for a, b in zip(*out):  # the same operations in the same order
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b)
