@@ -507,6 +507,8 @@ static DirectDiv direct_div(int n) {
     return {(unsigned)(((1ull << (31 + s)) / (unsigned)n) + 1), s};
 }
 
+constexpr int kGridRows = 65535;  // gridDim.y at most
+
 // Grid of the direct kernels: V cells and np planes per thread, 128 threads,
 // the field sets of a cell in threadIdx.y (as many as there are warps).
 // Returns whether both faces of an axis reach one cell.
@@ -535,7 +537,9 @@ static bool direct_grid(const StencilArgs<T>& a, DirectArgs& d, int V, dim3& gri
     }
     const int nset = std::min(a.B, kDirectThreads / 32);
     block = dim3(kDirectThreads / nset / 32 * 32, nset, 1);
-    if (d.np < 1) d.np = 1;
+    // one plane per thread, more on meshes with more planes than a grid has
+    // rows of blocks
+    d.np = std::max({1, d.np, (a.g.nx + kGridRows) / kGridRows});
     const AxisSlabs& z = d.ax[0][2];
     const int nvec = a.g.nz / V + 1;
     d.n_low = std::min(nvec, (z.n[0] + V - 1) / V);

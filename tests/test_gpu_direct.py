@@ -285,3 +285,21 @@ def test_dispersion_added_to_a_prepared_handle(where, form, precision):
             out.append((*eng.read_fields(), *eng.read_vi(), eng.read_dft(0, "Ex")))
     for a, b in zip(*out):  # the same operations in the same order
         assert np.all(np.isfinite(a)) and np.array_equal(a, b)
+
+
+@pytest.mark.parametrize("form", [None, ("fused", 16, 0)])
+def test_more_planes_than_one_grid_dimension(form):
+    """A long thin box of 70 001 planes, more than the 65 535 blocks of a
+    grid's y dimension: the direct kernels give the stream kernels' march."""
+    out = []
+    for f in (form, ("stream", 0, 0)):
+        prob = _problem((70000, 2, 3), (10, 10, 0, 0, 0, 0), "pec", 1)
+        with prob.build_engine("single") as eng:
+            if f:
+                eng.configure_stencil(*f)
+            eng.step(STEPS)
+            out.append((*eng.read_fields(), *eng.read_vi()))
+            assert eng.steps_done == STEPS
+    for q, (a, b) in enumerate(zip(*out)):
+        scale = float(np.max(np.abs(b)))
+        assert scale > 0 and float(np.max(np.abs(a - b))) <= (1 if q < 2 else 10) * TOL["single"] * scale, q
