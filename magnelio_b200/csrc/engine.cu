@@ -1297,7 +1297,9 @@ int enqueue_step(Handle& H) {
 int enqueue_step_any(Handle& H) { return H.prec == 4 ? enqueue_step<float>(H) : enqueue_step<double>(H); }
 
 // Captures nsteps steps starting from the current buffer set; the host-side
-// buffer set index is restored (the graph has not run yet).
+// buffer set index is restored (the graph has not run yet).  A launch that the
+// runtime refuses leaves no node and no error in the capture: it is asked for
+// here, so that no graph is kept that would march without it.
 cudaGraphExec_t capture(Handle& H, int nsteps, int* launches_per) {
     cudaGraph_t graph = nullptr;
     const int cur0 = H.cur;
@@ -1310,9 +1312,11 @@ cudaGraphExec_t capture(Handle& H, int nsteps, int* launches_per) {
     int per = 0;
     try {
         for (int s = 0; s < nsteps; ++s) per = enqueue_step_any(H);
+        ck(cudaGetLastError(), "step launch");
     } catch (...) {
         cudaStreamEndCapture(H.stream, &graph);
         if (graph) cudaGraphDestroy(graph);
+        cudaGetLastError();  // reported by the exception
         throw;
     }
     ck(cudaStreamEndCapture(H.stream, &graph), "end capture");
@@ -3085,6 +3089,7 @@ int fitb_time_stencil(fitb_handle* h, int32_t n_iter, double* ms_e, double* ms_h
             nl += fitb::launch_fused_any(H);
             if (!fitb::slab_in_place(H)) H.cur ^= 1;
         }
+        ck(cudaGetLastError(), "stencil launch");
         ck(cudaEventRecord(ev[1], H.stream), "event record");
         ck(cudaEventSynchronize(ev[1]), "event sync");
         H.launches += nl;
@@ -3100,6 +3105,7 @@ int fitb_time_stencil(fitb_handle* h, int32_t n_iter, double* ms_e, double* ms_h
     for (int q = 0; q < n_iter; ++q) fitb::launch_stencil_half(H, 0);
     ck(cudaEventRecord(ev[1], H.stream), "event record");
     for (int q = 0; q < n_iter; ++q) fitb::launch_stencil_half(H, 1);
+    ck(cudaGetLastError(), "stencil launch");
     ck(cudaEventRecord(ev[2], H.stream), "event record");
     ck(cudaEventSynchronize(ev[2]), "event sync");
     fitb::check_device_status(H);

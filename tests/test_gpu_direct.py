@@ -303,3 +303,45 @@ def test_more_planes_than_one_grid_dimension(form):
     for q, (a, b) in enumerate(zip(*out)):
         scale = float(np.max(np.abs(b)))
         assert scale > 0 and float(np.max(np.abs(a - b))) <= (1 if q < 2 else 10) * TOL["single"] * scale, q
+
+
+def test_a_form_that_cannot_launch_is_not_timed():
+    """One plane per CTA asks the stream kernels for more blocks than a grid's
+    z dimension has on a box of 70 001 planes: the stencil timer reports the
+    refused launches, and the step does."""
+    from magnelio_b200._lib import FitbError
+
+    prob = _problem((70000, 2, 3), (0,) * 6, "one", 1)
+    with prob.build_engine("single") as eng:
+        eng.configure_stencil("stream", 0, 1)
+        with pytest.raises(FitbError):
+            eng.time_stencil(2)
+        with pytest.raises(FitbError):
+            eng.step(1)
+        eng.configure_stencil("stream", 0, 0)
+        assert sum(eng.time_stencil(2)) > 0
+
+
+def test_a_step_that_cannot_launch_is_refused_every_time():
+    """A monitor whose phasors exceed a block's shared memory: no step may
+    count as done, on the first call or on any later one, timed or not, and
+    the handle without it steps on."""
+    from magnelio_b200._lib import FitbError
+    from magnelio_b200.problem import DftMonitor
+
+    prob = _problem((9, 8, 11), (0,) * 6, "one", 1)
+    with prob.build_engine("single") as eng:
+        eng.step(3)
+        want = eng.read_fields()
+    prob.monitors.append(DftMonitor(((0, 9), (0, 8), (5, 6)), ("Ez",), np.linspace(1e9, 9e9, 5000), 1))
+    with prob.build_engine("single") as eng:
+        for _ in range(2):
+            with pytest.raises(FitbError):
+                eng.step(3)
+            with pytest.raises(FitbError):
+                eng.step_timed(3)
+            assert eng.steps_done == 0
+    prob.monitors.pop()
+    with prob.build_engine("single") as eng:
+        eng.step(3)
+        assert all(np.array_equal(a, b) for a, b in zip(want, eng.read_fields()))
