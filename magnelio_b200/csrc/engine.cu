@@ -1511,7 +1511,7 @@ void set_form(Handle& H, int kind, int variant, int ichunk) {
     if (kind == kModeVec) H.vec_variant = variant;
     if (kind == kModeStream) H.stream_variant = compact ? 0 : variant;
     H.stencil_mode = kind;
-    H.direct_np = H.slab_ichunk = ichunk;
+    H.direct_np = H.slab_ichunk = std::min(ichunk, H.g.nx + 1);
     plan_stencil(H);
     if (ichunk > 0) {
         const int nplanes = H.g.nx + 1;

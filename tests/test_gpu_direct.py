@@ -345,3 +345,19 @@ def test_a_step_that_cannot_launch_is_refused_every_time():
     with prob.build_engine("single") as eng:
         eng.step(3)
         assert all(np.array_equal(a, b) for a, b in zip(want, eng.read_fields()))
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("depth", [1, 5, 54, 2**31 - 1])
+def test_planes_per_thread_of_the_direct_kernels(depth, precision):
+    """Any number of planes per thread, past the mesh too, gives the bits of
+    one plane per thread, and the handle reports no more planes than it has."""
+    out = []
+    for d in (0, depth):
+        prob = _problem((53, 53, 55), (6, 5, 4, 7, 5, 6), "pec", 1)
+        with prob.build_engine(precision) as eng:
+            eng.configure_stencil("simple", 0, d)
+            assert eng.stencil_config()["ichunk"] <= prob.nx + 1
+            eng.step(STEPS)
+            out.append((*eng.read_fields(), *eng.read_vi(), eng.read_dft(0, "Hz")))
+    assert all(np.array_equal(a, b) for a, b in zip(*out))
