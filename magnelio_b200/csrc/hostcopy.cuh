@@ -15,8 +15,8 @@
 
 #include <algorithm>
 #include <atomic>
+#include <exception>
 #include <functional>
-#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -55,9 +55,9 @@ struct HostLanes {
 
     // Reads `bytes` device bytes at `src` behind the work of stream `s`;
     // sink(offset, data, n) consumes the n bytes at `offset` and may run on
-    // several threads at once, on disjoint ranges.  Pieces are multiples of 16
-    // bytes.  Returns when every byte is consumed (or with the first error,
-    // after every thread has stopped).
+    // several threads at once, on disjoint ranges; it does not throw.  Pieces
+    // are multiples of 16 bytes.  Returns when every byte is consumed (or with
+    // the first error, after every thread has stopped).
     using Sink = std::function<void(size_t, const void*, size_t)>;
     cudaError_t read(int device, const void* src, size_t bytes, cudaStream_t s, const Sink& sink) {
         const size_t pieces = (bytes + kPiece - 1) / kPiece;
@@ -87,8 +87,8 @@ struct HostLanes {
         pool.reserve(lanes);
         try {
             for (int t = 1; t < lanes; ++t) pool.emplace_back(work, t);
-        } catch (const std::system_error&) {
-            // fewer threads than asked for: the others take their pieces
+        } catch (const std::exception&) {
+            // no thread or no memory for one: the others take its pieces
         }
         work(0);
         for (auto& t : pool) t.join();
