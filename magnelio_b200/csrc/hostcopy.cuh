@@ -67,6 +67,9 @@ struct HostLanes {
             cudaGetLastError();
             return read_pageable(src, bytes, s, sink);
         }
+        // one wait for the steps still queued: the threads spin in theirs
+        const cudaError_t rc = cudaStreamSynchronize(s);
+        if (rc != cudaSuccess) return rc;
         std::atomic<size_t> next{0};
         std::atomic<int> err{0};
         const auto work = [&](int lane) {

@@ -1,6 +1,7 @@
 // Stand-in for the few CUDA runtime calls of csrc/hostcopy.cuh, for
 // tests/hostcopy_check.cpp (included there as <cuda_runtime.h>): "device"
-// memory is host memory, copies happen at once, the n-th can be made to fail.
+// memory is host memory, copies happen at once, waits and the order of calls
+// are counted.
 #pragma once
 #include <atomic>
 #include <cstdlib>
@@ -13,11 +14,11 @@ typedef int* cudaEvent_t;
 constexpr unsigned cudaEventDisableTiming = 2;
 
 namespace fake {
-inline std::atomic<int> copies{0};
+inline std::atomic<int> waits{0}, copies{0}, copies_before_wait{0};
 inline bool no_pinned = false;
 inline long fail_copy = -1;  // index of the copy that fails
 inline void reset() {
-    copies = 0;
+    waits = copies = copies_before_wait = 0;
     no_pinned = false;
     fail_copy = -1;
 }
@@ -44,8 +45,12 @@ inline cudaError_t cudaEventDestroy(cudaEvent_t e) {
 }
 inline cudaError_t cudaEventRecord(cudaEvent_t, cudaStream_t) { return cudaSuccess; }
 inline cudaError_t cudaEventSynchronize(cudaEvent_t) { return cudaSuccess; }
-inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }
+inline cudaError_t cudaStreamSynchronize(cudaStream_t) {
+    ++fake::waits;
+    return cudaSuccess;
+}
 inline cudaError_t cudaMemcpyAsync(void* dst, const void* src, size_t n, cudaMemcpyKind, cudaStream_t) {
+    if (fake::waits == 0) ++fake::copies_before_wait;
     if (fake::copies++ == fake::fail_copy) return cudaErrorUnknown;
     std::memcpy(dst, src, n);
     return cudaSuccess;

@@ -1,9 +1,10 @@
 // CPU check of the threaded device-to-host reads (magnelio_b200/csrc/hostcopy.cuh)
 // against a stand-in CUDA runtime (a header of its own beside the compiled
 // copy of this file): every byte arrives once, at sizes around a piece and a
-// lane; a thread that cannot be created for want of memory leaves its pieces
-// to the others; a missing page-locked allocation and a failing copy behave as
-// documented.
+// lane; the stream's queued work is waited for once, before any piece is
+// copied or any thread started; a thread that cannot be created, for want of
+// a thread or of memory, leaves its pieces to the others; a missing
+// page-locked allocation and a failing copy behave as documented.
 #include <algorithm>
 #include <atomic>
 #include <cstdio>
@@ -53,6 +54,7 @@ static int run(size_t bytes, long allocs, bool no_pinned, long fail_copy) {
     if (threw) return 0;
     const bool twice = std::any_of(seen.begin(), seen.end(), [](const std::atomic<int>& c) { return c.load() > 1; });
     if (rc != cudaSuccess || twice || memcmp(src.data(), dst.data(), bytes)) return 1;
+    if (!no_pinned && bytes && (fake::waits != 1 || fake::copies_before_wait != 0)) return 2;
     return 0;
 }
 

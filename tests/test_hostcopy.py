@@ -1,7 +1,8 @@
 """The threaded device-to-host reads (host code, csrc/hostcopy.cuh): compiled
 with the host compiler against a stand-in CUDA runtime and checked by
-tests/hostcopy_check.cpp (every byte once, threads that cannot be created, no
-page-locked memory, a failing copy)."""
+tests/hostcopy_check.cpp (every byte once, one wait for the stream's queued
+work before the first piece, threads that cannot be created, no page-locked
+memory, a failing copy)."""
 
 from __future__ import annotations
 
