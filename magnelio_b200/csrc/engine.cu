@@ -269,6 +269,7 @@ struct Handle {
     int dft_blocks = 0;
     DftPack dft_pack{};
     size_t dft_smem = 0;
+    bool dft_one_launch = true;  // the monitors' staging and flush share a launch
     DevBuf ticket;  // CTA completion counter of the monitor launch
     int launches_per_step = 0;
     bool port_tables_dirty = true;
@@ -690,12 +691,14 @@ void refresh_port_tables(Handle& H) {
     upload(H.d_band, bd);
     // monitors: block ranges of the merged stage / flush launches
     std::vector<DftDev> dd;
+    H.dft_one_launch = true;
+    for (auto& m : H.dft) H.dft_one_launch = H.dft_one_launch && dft_one_launch(m->dev, H.B);
     int sb = 0;
     size_t smem = 0;
     for (auto& m : H.dft) {
         DftDev d = m->dev;
         d.sblk0 = sb;
-        d.sblk = fitb::dft_blocks((long long)d.ncomp * d.ncell);
+        d.sblk = fitb::dft_blocks((long long)H.B * d.ncomp * d.ncell, H.dft_one_launch);
         sb += d.sblk;
         smem = std::max(smem, (size_t)d.K * 2 * d.nf * sizeof(float2));
         m->dev.sblk0 = d.sblk0;
@@ -1221,10 +1224,9 @@ int enqueue_step_fused(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_step<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.dft_pack, H.d_dft.as<DftDev>(),
-                           (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), 0,
-                           H.ticket.as<unsigned>(), H.stream);
-        ++n;
+        n += launch_dft_step<T>(e_new, h_new, H.e_block(), H.e_block(), H.g, H.B, H.dft_pack, H.d_dft.as<DftDev>(),
+                                (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.dft_one_launch,
+                                H.step.as<long long>(), 0, H.ticket.as<unsigned>(), H.stream);
     } else {
         launch_advance(H.step.as<long long>(), H.stream);
         ++n;
@@ -1283,10 +1285,9 @@ int enqueue_step(Handle& H) {
         ++n;
     }
     if (!H.dft.empty()) {
-        launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.dft_pack,
-                           H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.step.as<long long>(), advance ? 1 : 0,
-                           H.ticket.as<unsigned>(), H.stream);
-        ++n;
+        n += launch_dft_step<T>(H.Ec().as<T>(), H.Hc().as<T>(), H.e_block(), H.e_block(), H.g, H.B, H.dft_pack,
+                                H.d_dft.as<DftDev>(), (int)H.dft.size(), H.dft_blocks, H.dft_smem, H.dft_one_launch,
+                                H.step.as<long long>(), advance ? 1 : 0, H.ticket.as<unsigned>(), H.stream);
     } else if (!advance) {
         launch_advance(H.step.as<long long>(), H.stream);
         ++n;

@@ -486,19 +486,22 @@ struct DftDev {
     int sblk0, sblk;      // this monitor's blocks in the merged launch
 };
 
-int dft_blocks(long long work);
-// One launch per step stages every monitor's samples and flushes the full
-// ones (dynamic shared memory for the largest monitor's phasors).  done = 1:
-// the step counter is already advanced; 0: this launch advances it (its last
-// CTA, through `ticket`).
+// Whether a monitor may share the launch that stages and flushes (a sample of
+// one field set per thread), and the CTAs of one of `work` samples per step.
+bool dft_one_launch(const DftDev& d, int B);
+int dft_blocks(long long work, bool one_launch);
+// Stages every monitor's samples and flushes the full ones, in one launch
+// (where every monitor allows it) or two; returns their number.  smem: dynamic
+// shared memory for the largest monitor's phasors.  done = 1: the step counter
+// is already advanced; 0: advanced here (by the last CTA, through `ticket`).
 constexpr int kDftPack = 8;
 struct DftPack {
     DftDev d[kDftPack];  // the first monitors, as in the device table `devs`
 };
 template <typename T>
-void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                     const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step, int done,
-                     unsigned* ticket, cudaStream_t s);
+int launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
+                    const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, bool one_launch,
+                    long long* step, int done, unsigned* ticket, cudaStream_t s);
 // Host-requested flush of the first kc slots of one monitor.
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s);
 

@@ -12,8 +12,12 @@
 // samples forms sum_s w_s[f] x_s for every bin of that cell in registers and
 // adds it once to the bins (optionally Kahan-compensated): the complex bins
 // are read and written once per K recorded steps instead of once per step.
-// All monitors share this one launch per step (k_dft_step).
+// All monitors share one launch per step (k_dft_step), or, where one of them
+// has many samples, a launch that stages and one that flushes.
 #include "fitb_common.cuh"
+
+#include <algorithm>
+#include <type_traits>
 
 namespace fitb {
 
@@ -21,6 +25,7 @@ namespace {
 
 constexpr int kMaxK = 32;
 constexpr int kThreads = 256;
+constexpr int kResident = 148 * 4;  // CTAs of 64 registers a thread that the chip holds
 
 __device__ __forceinline__ long long recorded_upto(long long x, int stride) {
     // Number of steps n' in [0, x] with n' % stride == 0 (0 for x < 0).
@@ -76,25 +81,30 @@ __device__ __forceinline__ int monitor_of_block(const DftDev* devs, int nmon) {
 }
 
 // Adds kc staged samples x[s * xs] (s < n_st) and, at s = kc - 1, `last` to
-// the bins of one cell-component: bins bi + f * ncell, phasors sw.
+// the bins of one cell-component: bins bi + f * ncell, phasors sw.  FULL: a
+// block of kMaxK samples (up to 96 frequencies), whose sums need no comparison
+// per sample and frequency (six components of 0.9 M cells, 64 frequencies: 159
+// us per step against 254 with them).
+template <bool FULL>
 __device__ __forceinline__ void flush_cell(const DftDev& d, int kc, int tsel, const float* x, long long xs, int n_st,
                                            float last, long long bi, const float2* sw) {
     float v[kMaxK];
 #pragma unroll
     for (int s = 0; s < kMaxK; ++s) v[s] = s < n_st ? x[s * xs] : (s == kc - 1 ? last : 0.0f);
-    for (int f = 0; f < d.nf; ++f, bi += d.ncell) {
+    sw += tsel * d.nf;
+    for (int f = 0; f < d.nf; ++f, bi += d.ncell, ++sw) {
+        float2 acc = d.bins[bi], cm;
+        if (d.kahan) cm = d.cmp[bi];
         float re = 0.0f, im = 0.0f;
 #pragma unroll
         for (int s = 0; s < kMaxK; ++s) {
-            if (s < kc) {
-                const float2 w = sw[(s * 2 + tsel) * d.nf + f];
+            if (FULL || s < kc) {
+                const float2 w = sw[s * 2 * d.nf];
                 re = fmaf(w.x, v[s], re);
                 im = fmaf(w.y, v[s], im);
             }
         }
-        float2 acc = d.bins[bi];
         if (d.kahan) {
-            float2 cm = d.cmp[bi];
             const float yr = re - cm.x, yi = im - cm.y;
             const float tr = acc.x + yr, ti = acc.y + yi;
             cm.x = (tr - acc.x) - yr;
@@ -110,17 +120,26 @@ __device__ __forceinline__ void flush_cell(const DftDev& d, int kc, int tsel, co
     }
 }
 
-// One step of every monitor.  The step counter is *step - done: done = 1 when
-// an earlier kernel of the step has advanced it; otherwise the last CTA of
-// this launch does, through `ticket`.  Staging and flushing were two launches
-// before, the second one empty on K - 1 of K steps: on a 97 x 104 x 89 mesh
-// with three planes of 16 frequencies the two cost 13 us per step.  The
-// launch is short, so its chain counts: up to kDftPack descriptors travel as
-// kernel arguments (else a block's first loads are a descriptor from HBM or
+// One step of every monitor: PARTS = both, or the staging and the flush as
+// launches of their own.  The step counter is *step - done: done = 1 when an
+// earlier kernel of the step has advanced it; otherwise the last CTA to finish
+// (of the flush) does, through `ticket`.
+// Both in one launch saves the flush's, which is empty on K - 1 of K steps, and
+// gives a thread one sample of one field set: on a 97 x 104 x 89 mesh with
+// three planes of 16 frequencies 4.9 us per step against 8.4 in two launches;
+// eight sets of a 64 x 56 plane with 64 frequencies 7.1 us against 16.7 (and 44
+// where a thread walked its cell's sets).  From about 0.6 M samples on, two
+// launches of loops that hold 64 registers each: the staging of a cell's sets
+// shares its indexing, and no CTA is too short for its descriptor's latency
+// (three components of 0.9 M cells, eight frequencies: 39 us with one field set
+// and 105 with four; as one launch 48 and 186).
+// The launch is short, so its chain counts: up to kDftPack descriptors travel
+// as kernel arguments (else a block's first loads are a descriptor from HBM or
 // L2, one after the other per monitor), and the slot arithmetic is 32-bit
 // while the step count is.
-template <typename T, bool PACK>
-__global__ void __launch_bounds__(kThreads, 3)
+constexpr int kStage = 1, kFlush = 2;
+template <typename T, int PARTS, bool PACK>
+__global__ void __launch_bounds__(kThreads, 4)
     k_dft_step(const T* __restrict__ e, const T* __restrict__ h, long long e_block, long long h_block, Geom g, int B,
                const __grid_constant__ DftPack pack, const DftDev* __restrict__ devs_dev, int nmon, long long* step,
                int done, unsigned* ticket) {
@@ -143,9 +162,11 @@ __global__ void __launch_bounds__(kThreads, 3)
             slot = (int)((cnt - 1) % d.K);
         }
         const bool flush = slot == d.K - 1;
-        // this step's phasors: for the later steps of the block, and (every
-        // CTA for itself) for the flush
-        if (lb == 0 || flush) {
+        // this step's phasors: for the flush to come, and, where it is in this
+        // launch, every CTA for itself
+        constexpr bool kBoth = PARTS == (kStage | kFlush);
+        const bool own = kBoth && flush;
+        if ((PARTS & kStage) && (lb == 0 || own)) {
             const double tE = (double)n * d.dt;
             const double tH = tE + 0.5 * d.dt;
             const double dtw = (double)d.stride * d.dt;
@@ -156,37 +177,60 @@ __global__ void __launch_bounds__(kThreads, 3)
                 sincos(d.omega[f] * t, &sn, &cs);
                 const float2 w = make_float2((float)(cs * dtw), (float)(sn * dtw));
                 const long long at = ((long long)slot * 2 + (q / d.nf)) * d.nf + f;
-                if (flush)
+                if (own)
                     sw[at] = w;
                 else
                     d.wst[at] = w;
             }
         }
-        if (flush) {
-            for (int q = threadIdx.x; q < (d.K - 1) * 2 * d.nf; q += blockDim.x) sw[q] = d.wst[q];
+        if ((PARTS & kFlush) && flush) {
+            for (int q = threadIdx.x; q < (kBoth ? d.K - 1 : d.K) * 2 * d.nf; q += blockDim.x) sw[q] = d.wst[q];
             __syncthreads();
         }
-        const int total = d.ncomp * (int)d.ncell;
-        for (int t = lb * kThreads + threadIdx.x; t < total; t += d.sblk * kThreads) {
-            const int ci = t / (int)d.ncell;
-            const int cell = t - ci * (int)d.ncell;
+        const int per_set = d.ncomp * (int)d.ncell;
+        const int t0 = lb * kThreads + threadIdx.x;
+        const auto sample = [&](int b, int r) {  // component and cell r of field set b
+            const int ci = r / (int)d.ncell;
+            const int cell = r - ci * (int)d.ncell;
             const int kk = cell % d.nk;
-            const int r = cell / d.nk;
-            const int jj = r % d.nj;
-            const int ii = r / d.nj;
-            const int c = d.comps[ci];
-            for (int b = 0; b < B; ++b) {
-                const float v = (float)interp_sample<T>(e + (long long)b * e_block, h + (long long)b * h_block, g.vol,
-                                                        g, d, c, d.i0 + ii, d.j0 + jj, d.k0 + kk);
-                float* x = d.stage + ((long long)b * d.K * d.ncomp + ci) * d.ncell + cell;
+            const int rr = cell / d.nk;
+            const int jj = rr % d.nj;
+            const int ii = rr / d.nj;
+            return (float)interp_sample<T>(e + (long long)b * e_block, h + (long long)b * h_block, g.vol, g, d,
+                                           d.comps[ci], d.i0 + ii, d.j0 + jj, d.k0 + kk);
+        };
+        const auto add = [&](int b, int r, int n_st, float last) {
+            const int ci = r / (int)d.ncell;
+            const auto go = [&](auto full) {
+                flush_cell<decltype(full)::value>(
+                    d, d.K, d.comps[ci] < 3 ? 0 : 1, d.stage + (long long)b * d.K * per_set + r, per_set, n_st, last,
+                    (long long)(b * d.ncomp + ci) * d.nf * d.ncell + (r - ci * (int)d.ncell), sw);
+            };
+            if (d.K == kMaxK)
+                go(std::true_type());
+            else
+                go(std::false_type());
+        };
+        if constexpr (kBoth) {
+            if (t0 < B * per_set) {
+                const int b = t0 / per_set, r = t0 - b * per_set;
+                const float v = sample(b, r);
                 if (flush)
-                    flush_cell(d, d.K, c < 3 ? 0 : 1, x, (long long)total, d.K - 1, v,
-                               ((long long)(b * d.ncomp + ci) * d.nf) * d.ncell + cell, sw);
+                    add(b, r, d.K - 1, v);
                 else
-                    x[(long long)slot * total] = v;
+                    d.stage[((long long)b * d.K + slot) * per_set + r] = v;
+            }
+        } else if constexpr (PARTS == kStage) {
+            for (int r = t0; r < per_set; r += d.sblk * kThreads)
+                for (int b = 0; b < B; ++b) d.stage[((long long)b * d.K + slot) * per_set + r] = sample(b, r);
+        } else if (flush) {
+            for (int t = t0; t < B * per_set; t += d.sblk * kThreads) {
+                const int b = t / per_set;
+                add(b, t - b * per_set, d.K, 0.0f);
             }
         }
     }
+    if (PARTS == kStage) return;
     if (done) return;
     // The last CTA to finish advances the step counter: every CTA has read
     // it above, and the next launch in the stream starts after this one.
@@ -213,41 +257,49 @@ __global__ void __launch_bounds__(kThreads) k_dft_flush_forced(int B, DftDev d, 
         const long long r = t % per_b;
         const int ci = (int)(r / d.ncell);
         const long long cell = r % d.ncell;
-        flush_cell(d, kc, d.comps[ci] < 3 ? 0 : 1, d.stage + ((long long)b * d.K * d.ncomp + ci) * d.ncell + cell,
+        flush_cell<false>(d, kc, d.comps[ci] < 3 ? 0 : 1, d.stage + ((long long)b * d.K * d.ncomp + ci) * d.ncell + cell,
                    per_b, kc, 0.0f, ((long long)(b * d.ncomp + ci) * d.nf) * d.ncell + cell, sw);
     }
 }
 
 }  // namespace
 
-int dft_blocks(long long work) {
-    long long b = (work + kThreads - 1) / kThreads;
-    if (b > 148 * 4) b = 148 * 4;
-    return (int)(b < 1 ? 1 : b);
+bool dft_one_launch(const DftDev& d, int B) {
+    return (long long)B * d.ncomp * d.ncell <= 4LL * kResident * kThreads;
+}
+
+int dft_blocks(long long work, bool one_launch) {
+    const long long n = (work + kThreads - 1) / kThreads;
+    return (int)std::max(1LL, one_launch ? n : std::min<long long>(n, kResident));
 }
 
 template <typename T>
-void launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
-                     const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, long long* step,
-                     int done, unsigned* ticket, cudaStream_t s) {
-    if (nmon <= kDftPack)
-        k_dft_step<T, true>
-            <<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, pack, devs, nmon, step, done, ticket);
-    else
-        k_dft_step<T, false>
-            <<<nblocks, kThreads, smem, s>>>(e, h, e_block, h_block, g, B, pack, devs, nmon, step, done, ticket);
+int launch_dft_step(const T* e, const T* h, long long e_block, long long h_block, const Geom& g, int B,
+                    const DftPack& pack, const DftDev* devs, int nmon, int nblocks, size_t smem, bool one_launch,
+                    long long* step, int done, unsigned* ticket, cudaStream_t s) {
+    const auto go = [&](auto k, size_t sm) {
+        k<<<nblocks, kThreads, sm, s>>>(e, h, e_block, h_block, g, B, pack, devs, nmon, step, done, ticket);
+    };
+    const bool packed = nmon <= kDftPack;
+    if (one_launch) {
+        packed ? go(k_dft_step<T, kStage | kFlush, true>, smem) : go(k_dft_step<T, kStage | kFlush, false>, smem);
+        return 1;
+    }
+    packed ? go(k_dft_step<T, kStage, true>, 0) : go(k_dft_step<T, kStage, false>, 0);
+    packed ? go(k_dft_step<T, kFlush, true>, smem) : go(k_dft_step<T, kFlush, false>, smem);
+    return 2;
 }
 
 void launch_dft_flush_forced(int B, const DftDev& d, int kc, cudaStream_t s) {
     const size_t smem = (size_t)kc * 2 * d.nf * sizeof(float2);
-    k_dft_flush_forced<<<dft_blocks((long long)B * d.ncomp * d.ncell), kThreads, smem, s>>>(B, d, kc);
+    k_dft_flush_forced<<<dft_blocks((long long)B * d.ncomp * d.ncell, false), kThreads, smem, s>>>(B, d, kc);
 }
 
-template void launch_dft_step<float>(const float*, const float*, long long, long long, const Geom&, int,
-                                     const DftPack&, const DftDev*, int, int, size_t, long long*, int, unsigned*,
-                                     cudaStream_t);
-template void launch_dft_step<double>(const double*, const double*, long long, long long, const Geom&, int,
-                                      const DftPack&, const DftDev*, int, int, size_t, long long*, int, unsigned*,
-                                      cudaStream_t);
+#define FITB_INST(T)                                                                                                \
+    template int launch_dft_step<T>(const T*, const T*, long long, long long, const Geom&, int, const DftPack&,      \
+                                    const DftDev*, int, int, size_t, bool, long long*, int, unsigned*, cudaStream_t);
+FITB_INST(float)
+FITB_INST(double)
+#undef FITB_INST
 
 }  // namespace fitb

@@ -361,3 +361,48 @@ def test_planes_per_thread_of_the_direct_kernels(depth, precision):
             eng.step(STEPS)
             out.append((*eng.read_fields(), *eng.read_vi(), eng.read_dft(0, "Hz")))
     assert all(np.array_equal(a, b) for a, b in zip(*out))
+
+
+@pytest.mark.parametrize("precision", ["double", "single"])
+@pytest.mark.parametrize("n,batch,n_freq", [
+    ((9, 8, 11), 3, 5),        # a sample per thread, one launch
+    ((20, 19, 31), 8, 130),    # blocks of fewer than 32 steps
+    ((60, 62, 64), 1, 3),      # many samples: staging and flush as launches of their own
+    ((60, 62, 64), 2, 100),    # the same with short blocks and two field sets
+])
+def test_monitored_batches_equal_their_field_sets(n, batch, n_freq, precision):
+    """Volume monitors of a batch, over whole and partial slot blocks, on
+    meshes on both sides of the samples that one launch takes: every field
+    set's bins are those of a handle of its own, bit for bit, and the DFT sums
+    of the fields read after every step."""
+    from magnelio_b200.problem import DftMonitor
+
+    steps = 70
+    freqs = np.linspace(1e9, 9e9, n_freq)
+
+    def problem(sets):
+        prob = _problem(n, (0,) * 6, "one", batch)
+        prob.lumped = []
+        prob.e0, prob.h0 = [prob.e0[b] for b in sets], [prob.h0[b] for b in sets]
+        prob.batch = len(sets)
+        prob.monitors = [DftMonitor(tuple((0, v) for v in n), ("Ex", "Ey", "Hz"), freqs, 1)]
+        return prob
+
+    with problem(range(batch)).build_engine(precision) as eng:
+        eng.step(steps)
+        got = [[eng.read_dft(0, c, b) for c in ("Ex", "Ey", "Hz")] for b in range(batch)]
+    for b in range(batch):
+        prob = problem([b])
+        with prob.build_engine(precision) as eng:
+            shape, want = eng.shapes["Ex"], 0.0
+            for s in range(steps):
+                eng.step(1)
+                if b == 0 and n_freq <= 5:
+                    ex = eng.read_fields()[0][:int(np.prod(shape))].reshape(shape)
+                    cell = 0.25 * (ex[:, :-1, :-1] + ex[:, 1:, :-1] + ex[:, :-1, 1:] + ex[:, 1:, 1:])
+                    cell = cell / prob.dx[:, None, None]
+                    want = want + np.exp(2j * np.pi * freqs * s * prob.dt)[:, None, None, None] * prob.dt * cell
+            one = [eng.read_dft(0, c) for c in ("Ex", "Ey", "Hz")]
+        assert all(np.array_equal(x, y) for x, y in zip(got[b], one))
+        if b == 0 and n_freq <= 5:
+            assert np.max(np.abs(one[0] - want)) <= 1e-5 * np.max(np.abs(want))  # float32 samples and bins
