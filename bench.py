@@ -733,8 +733,7 @@ def run_b200(args, world, rank, local):
     peak, peak_kind = _peaks()
     tile = stencil_cfg["kind"] == "fused" and TILE_VARIANT_BASE <= stencil_cfg["variant"] < SLAB_VARIANT_BASE
     slab = stencil_cfg["kind"] == "fused" and stencil_cfg["variant"] >= SLAB_VARIANT_BASE
-    # the slab step without a given march depth runs on the direct kernels
-    lists = slab and tuned is not None and tuned.ichunk > 0
+    lists = slab and stencil_cfg["ichunk"] > 0  # 0: the slab step runs on the direct kernels
     if lists:
         kernel = "k_step_slab (one stencil step, CPML inside the march)"
         traffic = _traffic("slab_step", n, cpml_cells) if B == 1 else None

@@ -222,8 +222,9 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind);
  * precision, dispersion or CPML layout does not take), and the number of i
  * planes one CTA marches (0: the form's own plan).  The fields, psi and all
  * other state carry over; valid between steps.
- * fitb_get_stencil writes kind, variant, planes per CTA and the grid
- * (x, y, z) into out[6]. */
+ * fitb_get_stencil writes kind, variant, and the planes per CTA and grid
+ * (x, y, z) of the kernels that step it into out[6]; 0 planes for a slab step
+ * that runs on the direct kernels (configured with 0 it does so again). */
 #define FITB_STENCIL_SIMPLE 0
 #define FITB_STENCIL_STREAM 1
 #define FITB_STENCIL_BULK 2

@@ -49,6 +49,9 @@ struct DirectArgs {
 // which: 0 = E update, 1 = H update
 template <typename T>
 void launch_direct_half(const StencilArgs<T>& a, const DirectArgs& d, int which, cudaStream_t s);
+// Planes per thread and grid (x, y, z) of those launches for np (0: their own).
+template <typename T>
+void direct_shape(const StencilArgs<T>& a, int np, int* out);
 // flags[side] (zeroed by the caller): bit 0 set when alpha is not (beta != 0),
 // bit 1 when it is not 1 everywhere.
 template <typename T>

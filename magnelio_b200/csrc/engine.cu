@@ -1435,6 +1435,38 @@ void run_steps(Handle& H, long long nsteps) {
     H.steps_done += nsteps;
 }
 
+// What fitb_get_stencil says: the form, and the depth and grid of the kernels
+// that step it.
+void report_form(Handle& H, int32_t* out) {
+    bool direct = H.stencil_mode == kModeSimple;
+    if (H.stencil_mode == kModeFused && is_slab_variant(H.fused_variant) && H.coeffs_set) {
+        try {
+            refresh_port_tables(H);  // the choice follows the unit lists
+            direct = !slab_on_lists(H);
+        } catch (const Error&) {
+            // lists that the next step will refuse
+        }
+    }
+    const bool planned =
+        H.stencil_mode == kModeStream || H.stencil_mode == kModeVec || H.stencil_mode == kModeFused;
+    out[0] = H.stencil_mode;
+    out[1] = H.stencil_mode == kModeVec     ? H.vec_variant
+             : H.stencil_mode == kModeFused ? H.fused_variant
+             : H.stencil_mode == kModeStream ? H.stream_variant
+                                             : 0;
+    out[2] = planned ? H.splan.ichunk : (H.stencil_mode == kModeBulk ? H.plan.ichunk : 0);
+    out[3] = planned ? H.splan.grid_x : 0;
+    out[4] = planned ? H.splan.grid_y : 0;
+    out[5] = planned ? H.splan.grid_z : 0;
+    if (direct) {
+        const int np = H.stencil_mode == kModeSimple ? H.direct_np : 0;
+        H.prec == 4 ? direct_shape(stencil_args<float>(H), np, out + 2)
+                    : direct_shape(stencil_args<double>(H), np, out + 2);
+        // a depth would move the slab step to its unit lists
+        if (H.stencil_mode == kModeFused) out[2] = 0;
+    }
+}
+
 // Switches the stencil form between steps.
 void set_form(Handle& H, int kind, int variant, int ichunk) {
     if (kind < kModeSimple || kind > kModeFused) fail(FITB_ERR_ARG, "stencil kind %d", kind);
@@ -2146,17 +2178,7 @@ int fitb_get_stencil(fitb_handle* h, int32_t* out) {
     FITB_TRY
     Handle& H = H_of(h);
     if (!out) fail(FITB_ERR_ARG, "null argument");
-    const bool planned = H.stencil_mode == fitb::kModeStream || H.stencil_mode == fitb::kModeVec ||
-                         H.stencil_mode == fitb::kModeFused;
-    out[0] = H.stencil_mode;
-    out[1] = H.stencil_mode == fitb::kModeVec     ? H.vec_variant
-             : H.stencil_mode == fitb::kModeFused ? H.fused_variant
-             : H.stencil_mode == fitb::kModeStream ? H.stream_variant
-                                                   : 0;
-    out[2] = planned ? H.splan.ichunk : (H.stencil_mode == fitb::kModeBulk ? H.plan.ichunk : std::max(1, H.direct_np));
-    out[3] = planned ? H.splan.grid_x : 0;
-    out[4] = planned ? H.splan.grid_y : 0;
-    out[5] = planned ? H.splan.grid_z : 0;
+    fitb::report_form(H, out);
     FITB_CATCH
 }
 

@@ -616,6 +616,18 @@ void launch_direct_half(const StencilArgs<T>& a0, const DirectArgs& d, int which
 }
 
 template <typename T>
+void direct_shape(const StencilArgs<T>& a, int np, int* out) {
+    DirectArgs d{};
+    d.np = np;
+    dim3 grid, block;
+    direct_grid<T>(a, d, direct_wide(a) ? 16 / (int)sizeof(T) : 1, grid, block);
+    out[0] = d.np;
+    out[1] = (int)grid.x;
+    out[2] = (int)grid.y;
+    out[3] = (int)grid.z;
+}
+
+template <typename T>
 void launch_unit_alpha(const StencilArgs<T>& a, int* flags, cudaStream_t s) {
     const dim3 grid(592, 6);
     if (a.coef_kind == kCoefF16)
@@ -652,6 +664,7 @@ void launch_energy(const T* e, const T* h, const T* meps, const T* mmu, const Ge
 
 #define FITB_INST(T)                                                                           \
     template void launch_direct_half<T>(const StencilArgs<T>&, const DirectArgs&, int, cudaStream_t); \
+    template void direct_shape<T>(const StencilArgs<T>&, int, int*);                           \
     template void launch_unit_alpha<T>(const StencilArgs<T>&, int*, cudaStream_t);             \
     template void launch_pack<T>(const T*, T*, const Geom&, int, long long, cudaStream_t);     \
     template void launch_unpack<T>(const T*, T*, const Geom&, int, long long, cudaStream_t);   \

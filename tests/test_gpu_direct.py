@@ -406,3 +406,26 @@ def test_monitored_batches_equal_their_field_sets(n, batch, n_freq, precision):
         assert all(np.array_equal(x, y) for x, y in zip(got[b], one))
         if b == 0 and n_freq <= 5:
             assert np.max(np.abs(one[0] - want)) <= 1e-5 * np.max(np.abs(want))  # float32 samples and bins
+
+
+def test_the_form_reported_is_the_form_that_runs():
+    """The slab step reports depth 0 and the direct kernels' grid where it runs
+    on them, its march depth where it runs on its unit lists, and what it
+    reports configures the same kernels again."""
+    prob = _problem((53, 53, 55), (6, 5, 4, 7, 5, 6), "one", 1)
+    with prob.build_engine("single") as eng:
+        default = eng.stencil_config()
+        assert default["kind"] == "simple" and default["ichunk"] == 1 and default["grid"][1] == prob.nx + 1
+        for depth in (0, 9):
+            eng.configure_stencil("fused", 18, depth)
+            cfg = eng.stencil_config()
+            assert (cfg["kind"], cfg["variant"], cfg["ichunk"]) == ("fused", 18, depth)
+            assert (cfg["grid"] == default["grid"]) == (depth == 0)
+            before = eng.launch_count
+            eng.step(1)
+            launches = eng.launch_count - before
+            eng.configure_stencil(cfg["kind"], cfg["variant"], cfg["ichunk"])
+            assert eng.stencil_config() == cfg
+            before = eng.launch_count
+            eng.step(1)
+            assert eng.launch_count - before == launches
