@@ -43,19 +43,22 @@ DEFAULT_CANDIDATES = (
     ("fused", 8, 0),
     ("fused", 9, 0),
     ("fused", 0, 0),
-    ("fused", 16, 0),
-    ("fused", 17, 0),
-    ("fused", 18, 0),
-    ("fused", 19, 0),
-    ("fused", 20, 0),
-    ("fused", 21, 0),
-    ("fused", 22, 0),
-    ("fused", 23, 0),
-    ("fused", 24, 0),
-    ("fused", 25, 0),
+    ("fused", 16, 0),  # the slab step's own choice: direct kernels or unit lists
+    # its unit lists
+    ("fused", 16, 16),
+    ("fused", 17, 16),
+    ("fused", 18, 16),
+    ("fused", 19, 16),
+    ("fused", 20, 16),
+    ("fused", 21, 16),
+    ("fused", 22, 16),
+    ("fused", 23, 16),
+    ("fused", 24, 16),
+    ("fused", 25, 16),
     ("bulk", 0, 0),
 )
-CANDIDATE_SET = 7  # bump when the candidates change: cached results of another set are not reused
+SLAB_VARIANT_BASE = 16  # fused variants from here on are the slab step
+CANDIDATE_SET = 8  # bump when the candidates change: cached results of another set are not reused
 
 
 @dataclass
@@ -111,25 +114,45 @@ def _store_cache(path: Path, key: str, res: TuneResult) -> None:
         pass  # a read-only home: tuning still works, it is just not remembered
 
 
+def _on_direct_kernels(eng, kind: str, variant: int) -> bool:
+    """Whether the form ``eng`` has just been given steps on the direct kernels."""
+    if kind == "simple":
+        return True
+    if kind != "default" and not (kind == "fused" and variant >= SLAB_VARIANT_BASE):
+        return False
+    cfg = eng.stencil_config()
+    return cfg["kind"] == "simple" or (cfg["kind"] == "fused" and cfg["ichunk"] == 0)
+
+
 def tune_engine(eng, candidates=DEFAULT_CANDIDATES, iters: int = 10, warmup: int = 2):
     """Time each candidate (kind, variant, ichunk) on ``eng`` and leave the
     fastest configured.  Candidates the handle refuses (a form that does not
-    take this batch width, a variant that does not fit) are skipped.  The
+    take this batch width, a variant that does not fit) are skipped, and so is
+    whatever runs on the direct kernels once they have been timed.
+    ``"default"`` is the handle as it comes, which no call configures again: it
+    is for the first candidate, and a scratch engine is not left on it.  The
     engine's fields advance: pass a scratch engine.  Returns (best, table)
     with per-candidate milliseconds for one E + H pass."""
     table = []
+    direct = False  # the direct kernels are timed
     for kind, variant, ichunk in candidates:
         try:
-            eng.configure_stencil(kind, variant, ichunk)
+            if kind != "default":
+                eng.configure_stencil(kind, variant, ichunk)
+            same = _on_direct_kernels(eng, kind, variant)
+            if same and direct:
+                continue
             eng.time_stencil(warmup)
             t_e, t_h = eng.time_stencil(iters)
         except FitbError:
             continue
         table.append((kind, int(variant), int(ichunk), float(t_e + t_h)))
+        direct = direct or same
     if not table:
         raise RuntimeError("no stencil candidate ran on this handle")
     best = min(table, key=lambda r: r[3])
-    eng.configure_stencil(best[0], best[1], best[2])
+    if best[0] != "default":
+        eng.configure_stencil(best[0], best[1], best[2])
     return best, table
 
 
@@ -157,6 +180,10 @@ def tune_problem(prob, precision: str = "single", batch_widths=(1,), device: int
     if getattr(prob, "dispersion", None):
         # the ADE update needs an in-place stencil form
         candidates = [c for c in candidates if c[0] != "fused"]
+    if coef != "native":
+        # the direct kernels take 16-bit coefficients on a handle that nobody
+        # configured, and no other way
+        candidates = [("default", 0, 0), *candidates]
     path = _cache_path()
     dev = _device_name(device)
     cache = _load_cache(path) if use_cache else {}
@@ -184,8 +211,10 @@ def tune_problem(prob, precision: str = "single", batch_widths=(1,), device: int
 
 
 def apply(eng, res: TuneResult) -> None:
-    """Configure a live engine with a tuning result (between steps)."""
-    eng.configure_stencil(res.kind, res.variant, res.ichunk)
+    """Configure a live engine with a tuning result (between steps); a new
+    engine is left as it comes where that was the fastest."""
+    if res.kind != "default":
+        eng.configure_stencil(res.kind, res.variant, res.ichunk)
 
 
 def best_batch(results) -> int:

@@ -95,3 +95,48 @@ def test_cache_keys_name_the_candidate_set():
     k = autotune.cache_key(64, 64, 64, 1, "single", "native", 6, "B200")
     assert k.endswith(f"|c{autotune.CANDIDATE_SET}")
     assert ("fused", 7, 0) in autotune.DEFAULT_CANDIDATES  # the tile form is tuned
+
+
+class SlabEngine(ScriptedEngine):
+    """A slab step without a depth runs on the direct kernels; 16-bit storage
+    refuses "simple"."""
+
+    def stencil_config(self):
+        kind, variant, ichunk = self.cfg or ("simple", 0, 0)
+        return {"kind": kind, "variant": variant, "ichunk": ichunk}
+
+    def time_stencil(self, n):
+        self.timed = [*getattr(self, "timed", []), self.cfg]
+        return super().time_stencil(n)
+
+
+def test_the_same_kernels_are_timed_once():
+    cands = [("simple", 0, 0), ("fused", 16, 0), ("fused", 17, 0), ("fused", 16, 16)]
+    times = {("simple", 0, 0): 1.0, ("fused", 16, 0): 0.99, ("fused", 17, 0): 0.98, ("fused", 16, 16): 2.0}
+    eng = SlabEngine(times)
+    best, table = autotune.tune_engine(eng, cands)
+    assert [r[:3] for r in table] == [("simple", 0, 0), ("fused", 16, 16)] and best[0] == "simple"
+    # where "simple" is refused, the first slab step stands for them
+    eng = SlabEngine(times, refuse={("simple", 0, 0)})
+    best, table = autotune.tune_engine(eng, cands)
+    assert [r[:3] for r in table] == [("fused", 16, 0), ("fused", 16, 16)] and best[:2] == ("fused", 16)
+
+
+def test_every_default_candidate_runs_kernels_of_its_own():
+    slabs = [c for c in autotune.DEFAULT_CANDIDATES if c[0] == "fused" and c[1] >= autotune.SLAB_VARIANT_BASE]
+    assert [c for c in slabs if c[2] == 0] == [("fused", 16, 0)]
+    assert {c[1] for c in slabs if c[2] > 0} == set(range(16, 26))  # the unit lists are tuned
+
+
+def test_sixteen_bit_coefficients_are_tuned_against_the_handle_as_it_comes(tmp_path, monkeypatch):
+    monkeypatch.setenv("FITB_TUNE_CACHE", str(tmp_path / "tune.json"))
+    eng = SlabEngine({None: 0.5, ("stream", 0, 0): 1.0, ("vec", 3, 0): 2.0}, refuse={("simple", 0, 0)})
+    monkeypatch.setattr(autotune, "_scratch_engine", lambda *a: eng)
+    cands = [("simple", 0, 0), ("stream", 0, 0), ("vec", 3, 0)]
+    res = autotune.tune_problem(_Prob(), coef="bf16", candidates=cands)
+    assert res.config() == ("default", 0, 0) and len(res.table) == 3
+    fresh = ScriptedEngine({})
+    autotune.apply(fresh, res)
+    assert fresh.log == []
+    native = autotune.tune_problem(_Prob(), candidates=cands, use_cache=False)
+    assert native.kind == "stream"
