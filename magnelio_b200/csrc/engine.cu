@@ -990,20 +990,48 @@ bool cpml_as_passes(const Handle& H, int side) {
     return !(H.stencil_mode == kModeSimple && H.coef_kind == kCoefNative && H.disp_clear[side]);
 }
 
-// The slab step (fused 16-25) on the direct kernels.  They are faster than
-// its unit lists at every size measured (float32, CPML all round, us per
-// step, lists / direct: 60 / 23 at 0.9 M cells, 280 / 200 at 10.9 M, 415 /
-// 310 at 16.8 M, 1119 / 840 at 49 M), with the same bits.  The lists stay
-// where the caller gave a march depth, and where more than kDeadShare of the
-// units are dead, which the lists leave out (a cross junction with 808 of
-// 1200 units dead steps on its lists at 84 Gcell/s of the dense mesh; the
-// direct kernels reach 56).
-constexpr double kDeadShare = 0.3;
+// The slab step (fused 16-25) on its unit lists or on the direct kernels, which
+// step the same fields to the same bits: whichever costs less, in units of the
+// direct kernels' time for a cell clear of CPML on a large mesh.  The lists cost
+//   kListsFixed                  five launches and their tails
+//   clear cells x 1.10           float32, one field set (96 B per cell and halos);
+//                 0.98, 1.01     batches, from eight sets on (one pass over the
+//                                fields, coefficients shared through the L2), 0.03
+//                                less where a CTA marches several sets;
+//                 0.95           16-bit coefficients;  1.12  float64
+//   cells of units with CPML x 1.95 (batches 1.70), a tenth less with 16 bits
+// and nothing for dead units; the direct kernels cost 1 for every cell, dead or
+// not, 0.25 more in units with CPML, and where alpha is read (the lists always
+// read it) 0.13 / sets more, 0.07 / sets in 16 bits, 0.12 + 0.14 / sets in
+// float64.  us per step, lists / direct: 290 / 263
+// at 256^3 clear of CPML, 393 / 298 with eight layers all round, 919 / 993 and
+// 833 / 983 with four sets (shared CTA; float32, float16); 97 x 104 x 89: 21.8 /
+// 14.0 and 52.9 / 22.9; with half the mesh frozen 164 / 262 and 307 / 297 at
+// 256^3, 14.4 / 14.0 and 52.7 / 22.8; lossy 287 / 298 and 390 / 332 at 256^3.
+// Over 400 such pairs (0.2 to 134 M cells in all sets, 1 to 8 sets, both storages,
+// float64, CPML none, z, all round, up to 0.7 of the mesh frozen, lossy) the
+// choice is within 6 % of the faster one everywhere.
+// A march depth given by the caller asks for the lists.
+constexpr double kListsFixed = 0.5e6;
 bool slab_on_lists(const Handle& H) {
     if (H.slab_ichunk > 0) return true;
-    int units = H.n_slab_dead;
-    for (int n : H.n_slab_units) units += n;
-    return H.n_slab_dead > kDeadShare * units;
+    double total = H.n_slab_dead, cpml = 0.0;
+    for (int q = 0; q < kSlabLists; ++q) {
+        total += H.n_slab_units[q];
+        if (q > 0) cpml += H.n_slab_units[q];
+    }
+    if (total <= 0.0) return false;
+    const double clear = H.n_slab_units[0] / total;
+    cpml /= total;
+    const double cells = (double)(H.g.nx + 1) * (H.g.ny + 1) * (H.g.nz + 1) * H.B;
+    const bool half = H.coef_kind != kCoefNative, shared = slab_nb_of(H.fused_variant - kFusedSlabBase) > 1;
+    const double w_clear = H.prec == 8 ? 1.12
+                           : half      ? 0.95
+                           : H.B == 1  ? 1.10
+                                       : (H.B < 8 ? 0.98 : 1.01) - (shared ? 0.03 : 0.0);
+    const double w_cpml = (H.B == 1 ? 1.95 : 1.70) * (half ? 0.9 : 1.0);
+    const double alpha = H.unit_alpha ? 0.0 : (H.prec == 8 ? 0.12 + 0.14 / H.B : (half ? 0.07 : 0.13) / H.B);
+    return kListsFixed / cells + w_clear * clear + w_cpml * cpml < 1.0 + alpha + 0.25 * cpml;
 }
 // In place, in the current buffer set, where nothing stands between the E and
 // the H update but lumped ports that step inside the E kernel; else from one

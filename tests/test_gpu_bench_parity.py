@@ -32,8 +32,9 @@ FIELD_TOL = 2e-4     # ||x - x_ref|| / max_n ||x_ref(n)||, float32 engine vs flo
 DFT_TOL = 2e-3       # max |bin - bin_ref| / max |bin_ref| per monitor component
 DFT_L2_TOL = 5e-4    # ||bins - bins_ref|| / ||bins_ref|| per monitor component
 
-# two-pass stream kernels, TMA tile step with CPML passes, slab step (CPML inside the march)
-FORMS = [("stream", 0), ("fused", 7), ("fused", 16)]
+# two-pass stream kernels, TMA tile step with CPML passes, slab step on the direct
+# kernels, and on its unit lists (CPML inside the march)
+FORMS = [("stream", 0, 0), ("fused", 7, 0), ("fused", 16, 0), ("fused", 16, 16)]
 
 
 def _reference(n, steps):
@@ -54,14 +55,16 @@ def ref256():
     return _reference(256, 500)
 
 
-def _check(prob, ref, kind, variant):
+def _check(prob, ref, kind, variant, depth):
     with prob.build_engine("single") as eng:
-        eng.configure_stencil(kind, variant)
+        eng.configure_stencil(kind, variant, depth)
         assert eng.stencil_config()["kind"] == kind
+        if variant == 16:
+            assert eng.stencil_config()["ichunk"] == depth
         eng.step(ref.steps)
         e, h = eng.read_fields()
         par = ref.compare(e, h, eng.read_dft)
-    print(f"{prob.nx}^3 {kind}/{variant}: {par}")
+    print(f"{prob.nx}^3 {kind}/{variant}/{depth}: {par}")
     assert par["rel_l2_e"] < FIELD_TOL, par
     assert par["rel_l2_h"] < FIELD_TOL, par
     assert par["dft_max_rel"] < DFT_TOL, par
@@ -69,11 +72,11 @@ def _check(prob, ref, kind, variant):
     return par
 
 
-@pytest.mark.parametrize("kind,variant", FORMS)
-def test_brick_box_128_prefix_matches_float64(ref128, kind, variant):
-    _check(*ref128, kind, variant)
+@pytest.mark.parametrize("kind,variant,depth", FORMS)
+def test_brick_box_128_prefix_matches_float64(ref128, kind, variant, depth):
+    _check(*ref128, kind, variant, depth)
 
 
-@pytest.mark.parametrize("kind,variant", FORMS)
-def test_brick_box_256_prefix_matches_float64(ref256, kind, variant):
-    _check(*ref256, kind, variant)
+@pytest.mark.parametrize("kind,variant,depth", FORMS)
+def test_brick_box_256_prefix_matches_float64(ref256, kind, variant, depth):
+    _check(*ref256, kind, variant, depth)

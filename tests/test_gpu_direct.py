@@ -429,3 +429,44 @@ def test_the_form_reported_is_the_form_that_runs():
             before = eng.launch_count
             eng.step(1)
             assert eng.launch_count - before == launches
+
+
+@pytest.mark.parametrize("n,batch,frozen,layers,lists", [
+    ((97, 104, 89), 1, 0.0, 8, False),     # CPML all round
+    ((97, 104, 89), 1, 0.45, 8, False),    # dead units, but few of them clear of the CPML
+    ((60, 62, 64), 1, 0.7, 0, False),      # mostly dead, but too small for five launches
+    ((160, 160, 160), 1, 0.5, 0, True),    # half dead
+    ((128, 120, 128), 4, 0.25, 0, True),   # a quarter dead, in a batch
+])
+def test_slab_step_takes_the_cheaper_of_its_two_routes(n, batch, frozen, layers, lists):
+    """Far from the line on both sides the unit lists run where dead units and
+    batches pay for them, the direct kernels elsewhere; and the bits are those
+    of the other route."""
+    from magnelio_b200 import host
+    from magnelio_b200.engine import FitEngine
+    from magnelio_b200.problem import FACES
+
+    rng = np.random.default_rng(1)
+    out = []
+    for depth in (0, 16):
+        with FitEngine(*n, 1e-13, batch=batch) as eng:
+            a, b = np.ones(eng.n_E), np.full(eng.n_E, 0.1)
+            off = 0
+            for c in ("Ex", "Ey", "Ez"):
+                s = eng.shapes[c]
+                m = int(np.prod(s))
+                for v in (a, b):
+                    v[off:off + m].reshape(s)[:, :int(frozen * s[1])] = 0.0
+                off += m
+            eng.set_coefficients(a, b, np.ones(eng.n_H), np.full(eng.n_H, 0.1))
+            for face in FACES if layers else ():
+                d = np.full(n["xyz".index(face[0])], 1e-3)
+                eng.add_cpml(face, *host.cpml_tables(d, face, 1e-13, thickness_cells=layers), (None,) * 4)
+            eng.configure_stencil("fused", 16, depth)
+            assert (eng.stencil_config()["ichunk"] > 0) == (lists or depth > 0)
+            if not out:
+                e0, h0 = rng.standard_normal(eng.n_E) * (b != 0), rng.standard_normal(eng.n_H)
+            eng.set_fields(e0.astype(np.float32), h0.astype(np.float32), batch - 1)
+            eng.step(5)
+            out.append(eng.read_fields(batch - 1))
+    assert all(np.all(np.isfinite(x)) and np.array_equal(x, y) for x, y in zip(*out))

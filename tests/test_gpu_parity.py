@@ -42,6 +42,19 @@ def _peaks(name):
     return r.peak_e, r.peak_h
 
 
+LIST_DEPTH = 9  # a march depth asks the slab step for its unit lists; 0 leaves the choice to it
+
+
+def _assert_route(eng, depth):
+    """The unit lists run with a march depth, the direct kernels without one
+    (which these meshes are small enough for)."""
+    nx = eng.shapes["Ex"][0]
+    assert eng.stencil_config()["ichunk"] == min(depth, nx + 1)
+
+
+SLAB_VARIANTS = range(16, 24)
+
+
 def _run(name, precision, steps=None):
     p, d, n = load_golden(name)
     eng = p.build_engine(precision=precision)
@@ -115,12 +128,15 @@ def test_stencil_variants_agree(name):
     arithmetic."""
     p, d, n = load_golden(name)
     outs = []
-    modes = [("stream", v) for v in range(4)] + [("bulk", 0), ("simple", 0)]
-    modes += [("vec", v) for v in range(4)] + [("fused", v) for v in range(24)]
-    for kind, variant in modes:
+    modes = [("stream", v, 0) for v in range(4)] + [("bulk", 0, 0), ("simple", 0, 0)]
+    modes += [("vec", v, 0) for v in range(4)] + [("fused", v, 0) for v in range(24)]
+    modes += [("fused", v, LIST_DEPTH) for v in SLAB_VARIANTS]  # the slab step's unit lists
+    for kind, variant, depth in modes:
         with p.build_engine("single") as eng:
-            eng.configure_stencil(kind, variant)
+            eng.configure_stencil(kind, variant, depth)
             assert eng.stencil_config()["kind"] == kind
+            if kind == "fused" and variant in SLAB_VARIANTS:
+                _assert_route(eng, depth)
             eng.step(n)
             outs.append(eng.read_fields())
     pe, ph = _peaks(name)
@@ -524,6 +540,38 @@ def test_fused_buffer_swaps_are_invisible(name, variant, monkeypatch):
         assert np.array_equal(ea, ec) and np.array_equal(ha, hc)
 
 
+@pytest.mark.parametrize("name", ["cpml_box", "mixed_box", "lumped_dft", "wg_dtbc", "wg_mur", "planewave_box"])
+@pytest.mark.parametrize("precision,tol", [("double", F64_TOL), ("single", F32_TOL)])
+@pytest.mark.parametrize("variant", [16, 17])
+def test_slab_unit_lists_match_reference(name, precision, tol, variant):
+    """The slab step on its unit lists reproduces the reference march: fields,
+    port V/I, DFT bins; odd and even step counts and a resume at an odd step
+    give the same bits."""
+    pe, ph = _peaks(name)
+    p, d, n = load_golden(name)
+    k = 2 * (n // 4) + 1  # odd
+    with p.build_engine(precision) as eng, p.build_engine(precision) as two, p.build_engine(precision) as res:
+        for q in (eng, two, res):
+            q.configure_stencil("fused", variant, LIST_DEPTH)
+            _assert_route(q, LIST_DEPTH)
+        eng.step(n)
+        e, h = eng.read_fields()
+        assert _rel(e, d["out.e"], pe) < tol
+        assert _rel(h, d["out.h"], ph) < tol
+        if "out.V" in d:
+            V, I = eng.read_vi()
+            assert _rel(V, d["out.V"]) < tol
+            assert _rel(I, d["out.I"]) < tol
+        for q, mon in enumerate(p.monitors):
+            for c in mon.components:
+                assert _rel(eng.read_dft(q, c), d[f"out.mon{q}.{c}"]) < max(5 * tol, DFT_TOL), (q, c)
+        two.step(k)
+        res.state_import(two.state_export())
+        for other in (two, res):
+            other.step(n - k)
+            assert all(np.array_equal(a, b) for a, b in zip((e, h), other.read_fields()))
+
+
 @pytest.mark.parametrize("mode", ["simple", "bulk"])
 def test_dispersion_in_other_stencil_modes(mode, monkeypatch):
     """The ADE update with separate CPML passes works with every in-place
@@ -671,8 +719,9 @@ def test_slab_workload_built_on_the_host_matches_the_oracle(precision, tol):
         assert _rel(bins[q], m.bins["Ex"]) < max(5 * tol, DFT_TOL)
 
 
+@pytest.mark.parametrize("depth", [0, LIST_DEPTH])
 @pytest.mark.parametrize("precision,tol", [("double", F64_TOL), ("single", F32_TOL)])
-def test_slab_workload_in_the_slab_step_matches_the_oracle(precision, tol):
+def test_slab_workload_in_the_slab_step_matches_the_oracle(precision, tol, depth):
     """The precision workload (Lorentz ADE slab one cell short of the CPML,
     TF/SF plane wave, DFT planes) in the slab step: the ADE update runs on
     the new E after the step kernel and the H cells next to dispersive
@@ -684,7 +733,8 @@ def test_slab_workload_in_the_slab_step_matches_the_oracle(precision, tol):
     n = 260
     ref = OracleRun(p).run(n)
     with p.build_engine(precision) as eng:
-        eng.configure_stencil("fused", 16)
+        eng.configure_stencil("fused", 16, depth)
+        _assert_route(eng, depth)
         eng.step(n)
         e, h = eng.read_fields()
         bins = [eng.read_dft(q, "Ex") for q in range(len(p.monitors))]
@@ -705,14 +755,17 @@ def test_slab_step_with_e_and_h_dispersion_matches_the_in_place_kernels(precisio
     p.cpml = []
     assert {x.side for x in p.dispersion} == {"E", "H"}
     outs = []
-    for kind, v in (("simple", 0), ("fused", 16)):
+    for kind, v, depth in (("simple", 0, 0), ("fused", 16, 0), ("fused", 16, LIST_DEPTH)):
         with p.build_engine(precision) as eng:
-            eng.configure_stencil(kind, v)
+            eng.configure_stencil(kind, v, depth)
+            if kind == "fused":
+                _assert_route(eng, depth)
             eng.step(n)
             outs.append(eng.read_fields())
     pe, ph = float(np.max(np.abs(outs[0][0]))), float(np.max(np.abs(outs[0][1])))
-    assert _rel(outs[1][0], outs[0][0], pe) < tol
-    assert _rel(outs[1][1], outs[0][1], ph) < tol
+    for e, h in outs[1:]:
+        assert _rel(e, outs[0][0], pe) < tol
+        assert _rel(h, outs[0][1], ph) < tol
 
 
 def test_slab_step_refuses_dispersion_inside_the_cpml():
@@ -826,7 +879,6 @@ def test_cross_junction_batch_equals_one_excitation_per_handle():
 # TMA tile form of the fused step on grids of many tiles and chunks.
 
 TILE_VARIANTS = range(7, 16)
-SLAB_VARIANTS = range(16, 24)
 
 
 def _random_state(prob, rng, scale=1e-3):
@@ -919,8 +971,9 @@ def test_slab_step_matches_stream_on_a_multi_tile_grid(n, precision, tol):
     assert ran >= (10 if precision == "single" else 6)
 
 
+@pytest.mark.parametrize("depth", [0, LIST_DEPTH])
 @pytest.mark.parametrize("variant", [16, 17])
-def test_slab_step_with_pec_masks_in_the_cpml(variant):
+def test_slab_step_with_pec_masks_in_the_cpml(variant, depth):
     """PEC air masks inside the CPML slabs (the air-mask boxes of the slab
     step), on a grid whose units see both faces of an axis (six-slot
     launches): fields match the reference march."""
@@ -929,7 +982,8 @@ def test_slab_step_with_pec_masks_in_the_cpml(variant):
         p, d, n = load_golden(name)
         assert any(a is not None and not np.all(a) for f in p.cpml for a in f.air)
         with p.build_engine("single") as eng:
-            eng.configure_stencil("fused", variant)
+            eng.configure_stencil("fused", variant, depth)
+            _assert_route(eng, depth)
             eng.step(n)
             e, h = eng.read_fields()
         assert _rel(e, d["out.e"], pe) < F32_TOL, name
@@ -990,7 +1044,8 @@ def test_slab_step_with_cpml_on_two_field_sets_matches_stream():
     assert not np.array_equal(outs["fused"][0][0], outs["fused"][1][0])
 
 
-def test_dead_units_are_skipped_bit_identically(monkeypatch):
+@pytest.mark.parametrize("depth", [0, LIST_DEPTH])
+def test_dead_units_are_skipped_bit_identically(depth, monkeypatch):
     """Dead-unit skipping (the reference's tile skip) on the four-port cross
     junction, whose PEC corner blocks freeze most of the grid: the slab step
     leaves the dead units out, and every field set's V/I and fields equal
@@ -1002,7 +1057,8 @@ def test_dead_units_are_skipped_bit_identically(monkeypatch):
     for skip in ("1", "0"):
         monkeypatch.setenv("FITB_TILE_SKIP", skip)
         with p.build_engine("single") as eng:
-            eng.configure_stencil("fused", 16)
+            eng.configure_stencil("fused", 16, depth)
+            _assert_route(eng, depth)
             units = eng.slab_units()
             eng.step(k)
             outs[skip] = ([eng.read_vi(b) for b in range(p.batch)], [eng.read_fields(b) for b in range(p.batch)],
@@ -1017,7 +1073,8 @@ def test_dead_units_are_skipped_bit_identically(monkeypatch):
         assert _rel(I, d[f"cross.I{b}"][:k]) < F32_TOL, b
 
 
-def test_dead_units_survive_a_resume_and_host_field_writes(monkeypatch):
+@pytest.mark.parametrize("depth", [0, LIST_DEPTH])
+def test_dead_units_survive_a_resume_and_host_field_writes(depth, monkeypatch):
     """A checkpoint resume into a skipping slab step, and fields written from
     the host with junk in the frozen cells: the skipped units' cells are made
     consistent across both buffer sets before the next step, so the
@@ -1026,14 +1083,14 @@ def test_dead_units_survive_a_resume_and_host_field_writes(monkeypatch):
     p, d, n = load_golden("cfg3_cross_small")
     k, m = 301, 200  # odd: the resume starts on the second buffer set
     with p.build_engine("single") as a:
-        a.configure_stencil("fused", 16)
+        a.configure_stencil("fused", 16, depth)
         a.step(k)
         blob = a.state_export()
         e_k, h_k = a.read_fields(3)
         a.step(m)
         ref = [a.read_fields(b) for b in range(p.batch)]
     with p.build_engine("single") as b_:
-        b_.configure_stencil("fused", 16)
+        b_.configure_stencil("fused", 16, depth)
         b_.state_import(blob)
         b_.step(m)
         got = [b_.read_fields(b) for b in range(p.batch)]
@@ -1049,7 +1106,7 @@ def test_dead_units_survive_a_resume_and_host_field_writes(monkeypatch):
     for skip in ("1", "0"):
         monkeypatch.setenv("FITB_TILE_SKIP", skip)
         with p.build_engine("single") as c:
-            c.configure_stencil("fused", 16)
+            c.configure_stencil("fused", 16, depth)
             c.state_import(blob)
             c.set_fields(e_junk, h_k, b=3)
             c.step(m)
