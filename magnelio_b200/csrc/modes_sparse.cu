@@ -58,8 +58,9 @@ __device__ double block_reduce(double x, double* sh) {
 
 // Barrier of all CTAs of a cooperative launch: `bar` counts arrivals (zeroed
 // before the launch), `round` is the caller's count of barriers so far.  The
-// wait is bounded; an expired one sets *err and every later barrier falls
-// through.
+// wait is bounded; an expired one sets *err to 1 and every later barrier falls
+// through.  (Another *err is no reason to leave: it may be set by a CTA that is
+// already past the barrier that this one still leaves.)
 constexpr unsigned kBarrierLimit = 1u << 24;
 __device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned& round, int* err) {
     __syncthreads();
@@ -70,7 +71,7 @@ __device__ __forceinline__ void grid_barrier(unsigned* bar, unsigned& round, int
         unsigned v, tries = 0;
         do {
             asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(bar) : "memory");
-        } while ((int)(v - target) < 0 && ++tries < kBarrierLimit && *(volatile int*)err == 0);
+        } while ((int)(v - target) < 0 && ++tries < kBarrierLimit && *(volatile int*)err != 1);
         if ((int)(v - target) < 0) atomicExch(err, 1);
         __threadfence();
     }
