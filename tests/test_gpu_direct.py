@@ -2,7 +2,10 @@
 stream kernels, which share none of their code: at the remainders of their
 16-byte cells and of a plane's threads, on both sides of the one-cell-per-thread
 bound, with slabs that overlap, masked or missing, for every way alpha can
-relate to beta, batch widths around a block's warps and the compact storages."""
+relate to beta, batch widths around a block's warps and the compact storages.
+The roundings are spelled out, so the bits agree; where the two slabs of an axis
+overlap, the direct kernels take all near faces before the far ones, another
+order of the corrections, and agree to rounding."""
 
 from __future__ import annotations
 
@@ -103,9 +106,11 @@ def test_direct_kernels_match_the_stream_kernels(n, layers, alpha, batch, precis
             want[1].append(vi[0])
             want = (want[0], want[1], want[2] or dft)
     tol = TOL[precision]
+    overlap = any(layers[2 * q] + layers[2 * q + 1] > n[q] for q in range(3))
 
     def close(a, b, scale, t):
         assert np.all(np.isfinite(a)) and float(np.max(np.abs(a - b))) <= t * scale
+        assert overlap or np.array_equal(a, b)
 
     for q in range(2):
         scale = max(float(np.max(np.abs(f[q]))) for f in want[0])
@@ -162,9 +167,8 @@ def test_cpml_stays_fused_beside_clear_dispersion(n, layers, precision):
                 eng.configure_stencil(form)
             eng.step(3 * max(n))
             out.append((*eng.read_fields(), *(eng.read_dft(m, "Ex") for m in range(2))))
-    for q, (a, b) in enumerate(zip(*out)):
-        scale = float(np.max(np.abs(b)))
-        assert scale > 0 and float(np.max(np.abs(a - b))) <= (TOL[precision] if q < 2 else 1e-5) * scale
+    for a, b in zip(*out):
+        assert float(np.max(np.abs(b))) > 0 and np.array_equal(a, b)
 
 
 def _slab_case(name, precision):
@@ -198,14 +202,12 @@ def test_slab_step_on_the_direct_kernels_matches_its_unit_lists(name, precision)
         prob = _slab_case(name, precision)
         with prob.build_engine(precision) as eng:
             eng.configure_stencil("fused", 16, depth)
+            assert (eng.stencil_config()["ichunk"] > 0) == (depth > 0)
             eng.step(20)
             eng.step(STEPS - 20)
             out.append([a for b in range(prob.batch) for a in (*eng.read_fields(b), *eng.read_vi(b))])
-    scale = [max(float(np.max(np.abs(a))) if a.size else 0.0 for a in out[1][q::4]) for q in range(4)]
     for q, (a, b) in enumerate(zip(*out)):
-        assert np.all(np.isfinite(a))
-        if a.size:
-            assert float(np.max(np.abs(a - b))) <= (1 if q % 4 < 2 else 10) * TOL[precision] * scale[q % 4], q
+        assert np.all(np.isfinite(a)) and np.array_equal(a, b), q
 
 
 @pytest.mark.parametrize("count", [1, 8, 9])
