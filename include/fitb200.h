@@ -210,8 +210,9 @@ int fitb_set_coeff_storage(fitb_handle* h, int32_t kind);
  * FITB_STENCIL_SIMPLE): kind FITB_STENCIL_SIMPLE / STREAM / BULK / VEC / FUSED,
  * a variant of that form (vec 0-3; fused 0-6 the register / cp.async forms,
  * fused 7-15 the TMA tile form with its CPML slab passes, tile shapes of
- * 2-16 rows x 32 cells and 3-5 ring stages; fused 16-25 the slab step, the
- * TMA tile march with the CPML inside it, tiles of 4, 2, 3, 4, 3, 2, 8, 6,
+ * 2-16 rows x 32 cells and 3-5 ring stages; fused 16-25 the slab step, on the
+ * direct kernels or, where a march depth is given or they cost less, on its unit
+ * lists, the TMA tile march with the CPML inside it, tiles of 4, 2, 3, 4, 3, 2, 8, 6,
  * 4, 4 rows x 32 cells with 3, 3, 3, 4, 4, 4, 3, 3, 3, 3 ring stages, one
  * field set per CTA except 24 and 25, which march 2 and 4 field sets per
  * CTA through shared coefficient boxes (the batch a multiple of that);

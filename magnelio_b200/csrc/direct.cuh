@@ -1,15 +1,11 @@
-// Arguments and launchers of the direct stencil kernels (stencil.cu): one
-// cell per thread, any number of field sets.
+// Arguments and launchers of the direct stencil kernels (stencil.cu): 16 bytes
+// of cells or one cell per thread, any number of field sets.
 #pragma once
 #include "fitb_common.cuh"
 
 namespace fitb {
 
-// What the direct kernels take beside StencilArgs (stencil.cu): the launcher
-// fills the division and the slab bounds, the caller the planes per thread,
-// the one-edge lumped ports that step inside the E kernel (their cell and
-// component; `ports` the device table in the same order) and the step counter
-// the H kernel advances (null: not advanced there).
+// One-edge lumped ports that may step inside the E kernel.
 constexpr int kDirectLumped = 16;
 // The CPML faces of one axis: [0] the layers 0 .. n[0] - 1, [1] the layers
 // lo1 .. lo1 + n[1] - 1 (lo1 = INT_MAX: none).  Entry of cell (i, j, k):
@@ -26,10 +22,16 @@ struct AxisSlabs {
     const void* bcc[2];
     const unsigned char* air[2];
 };
+// Division by a fixed n (direct_div).
 struct DirectDiv {
     unsigned m;
     int s;
 };
+// What the direct kernels take beside StencilArgs: the launcher fills the
+// division and the slab bounds, the caller the planes per thread (0: one), the
+// one-edge lumped ports that step inside the E kernel (their cell and
+// component; `ports` the device table in the same order) and the step counter
+// the H kernel advances (null: not advanced there).
 struct DirectArgs {
     int np;
     // vectors of a row: n_low in the near z slab, n_mid clear of both, n_edge

@@ -288,11 +288,12 @@ struct Handle {
     long long launches = 0;
     int direct_np = 0;  // planes per thread of the direct kernels (0: their own choice)
     // The stencil form is the engine's own choice, the direct kernels (no
-    // FITB_STENCIL, no fitb_configure_stencil): the fastest form at every
-    // size, batch and precision measured, from 8 us against the stream
-    // kernels' 41 us per step at 10 thousand cells to 1.82 ms against 2.56 ms
-    // (slab step: 2.25 ms) at 105 million.  It takes the compact coefficient
-    // storage, which an explicitly configured "simple" form refuses.
+    // FITB_STENCIL, no fitb_configure_stencil): faster than the stream kernels
+    // at every size, batch and precision measured, from 7.2 us against 88 us per
+    // step at 10 thousand cells (CPML all round) to 1.82 ms against 2.56 ms at
+    // 105 million; the slab step's unit lists, with a second buffer set, are
+    // faster on some large meshes (slab_on_lists).  It takes the compact
+    // coefficient storage, which an explicitly configured "simple" form refuses.
     bool auto_form = false;
     // alpha follows from beta (StencilArgs::unit_alpha) in the coefficients
     // as they are stored
@@ -967,11 +968,7 @@ void plan_stencil(Handle& H) {
     }
 }
 
-// One launch of the E (which == 0) or H (which == 1) update, with the
-// handle's kernel choice: the software-pipelined stencil for one field set,
-// the bulk-copy pipeline on request, the batched kernel for B > 1.  A side
-// with dispersive materials takes its CPML corrections in separate passes
-// after the ADE update, so its stencil launch carries no faces.
+// The lumped ports of a direct E launch that steps them (H.lumped_in_E).
 void direct_ports(Handle& H, const PortsArgs& pa, DirectArgs& da) {
     da.n_lumped = (int)H.lumped.size();
     for (int q = 0; q < da.n_lumped; ++q) da.lumped[q] = H.lumped_cell[q];
@@ -1041,9 +1038,11 @@ bool slab_in_place(const Handle& H) {
            H.modal.empty() && !H.disp[0].present() && !H.disp[1].present() && (H.lumped.empty() || H.lumped_in_E);
 }
 
-// In a step of the direct kernels, pa != null, the E launch steps the lumped
-// ports it can (H.lumped_in_E) and the H launch advances the step counter
-// when `advance` says so.
+// One launch of the E (which == 0) or H (which == 1) update of an in-place form.
+// A side whose CPML runs as passes launches without faces.  In a step of the
+// direct kernels, pa != null, the E launch steps the lumped ports it can
+// (H.lumped_in_E) and the H launch advances the step counter when `advance` says
+// so.
 template <typename T>
 void launch_half(Handle& H, int which, const PortsArgs* pa = nullptr, bool advance = false) {
     StencilArgs<T> sa = stencil_args<T>(H);
@@ -1362,7 +1361,7 @@ cudaGraphExec_t capture(Handle& H, int nsteps, int* launches_per) {
 // expired and the step's results are not valid.
 // the stencil forms whose copy pipelines record a status word
 bool has_device_status(const Handle& H) {
-    return H.stencil_mode == kModeBulk ||  (H.stencil_mode == kModeFused && H.fused_variant >= kFusedTileBase);
+    return H.stencil_mode == kModeBulk || (H.stencil_mode == kModeFused && H.fused_variant >= kFusedTileBase);
 }
 
 // error out on a nonzero status word `st` (read after the step), resetting it

@@ -101,7 +101,7 @@ template <typename T>
 void launch_compact(const T* src, unsigned short* dst, long long n, float inv_scale, int coef_kind, cudaStream_t s);
 
 // Software-pipelined register stencil, batched over B in {1, 2, 4, 8, 16}
-// field sets (the default kernels).
+// field sets (the stream form).
 struct StreamPlan {
     int ichunk;
     int grid_x, grid_y, grid_z;

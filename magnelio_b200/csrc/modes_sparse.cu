@@ -27,9 +27,10 @@
 // to fill the chip: the time is launches and host round trips.  So a filter
 // (up to 100 degrees) and the orthonormalisation of a block are one
 // cooperative launch each, their CTAs meeting at bounded grid barriers: on a
-// 104 x 46 plane with three modes the solve took 10.0 ms with a launch per
-// degree and some eight launches and two host reads per column, and 5.4 ms so
-// (7 iterations; 209 x 93: 15 ms).
+// 104 x 46 plane with three modes the solve took 8.5 ms with a launch per
+// degree and some eight launches and two host reads per column, and 4.8 ms so
+// (7 iterations; 209 x 93: 24 and 12.8 ms).  A call's allocations and frees come
+// on top and vary with what else the process holds (5 to 9 ms in all).
 #include "fitb_common.cuh"
 
 #include <algorithm>
@@ -308,7 +309,7 @@ int sparse_lowest_eigs(long long n, const long long* rp, const long long* col, c
     const size_t blk = (size_t)n * k;
     // five allocations of a few hundred KB rather than one: the driver serves
     // those from chunks it holds, while one of more than a MB is mapped and
-    // unmapped on every call (measured: 5.4 ms a solve against 8.6)
+    // unmapped on every call (measured: 5.4 ms a call against 8.6)
     double *X = nullptr, *Y = nullptr, *Yn = nullptr, *W = nullptr, *sm = nullptr;
     auto release = [&]() { cudaFree(X), cudaFree(Y), cudaFree(Yn), cudaFree(W), cudaFree(sm); };
     if (cudaMalloc(&X, blk * 8) || cudaMalloc(&Y, blk * 8) || cudaMalloc(&Yn, blk * 8) || cudaMalloc(&W, blk * 8) ||

@@ -1,5 +1,6 @@
 // Leapfrog curl updates with the CFS-PML psi recursion fused in: the direct
-// form, one cell per thread.
+// form, 16 bytes of cells per thread and no march (one cell per thread on small
+// meshes).
 //
 //   E^{n+1} = aE * E^n + bE * (C^T h)      then, on CPML slabs,
 //             E += +-bE * (ck * dH + psi_E),  psi_E = air * (b psi_E + c dH)
@@ -20,10 +21,10 @@
 // float32: latency and instructions bound them, not HBM) keep the whole chip
 // busy where a march along i (the stream, tile and slab forms) leaves most of
 // it idle; large meshes stream at the HBM rate (256^3 without CPML, float32:
-// 256 us per step, 96 B per cell at 0.98 of the measured copy rate).  Cells
-// per second, direct / stream / slab step: 36.8 / 14.4 / 15.0 G at 0.9 M cells,
-// 52 / 28 / 39 G at 10.9 M, 57.7 / 41.0 / 46.7 G at 105 M (CPML all round);
-// four field sets of 8 M cells 55 / 40 / 42 G.
+// 262 us per step, 96 B per cell at 0.95 of the measured copy rate).  Cells
+// per second, direct / stream / slab step's lists: 39 / 14.5 / 17.0 G at 0.9 M
+// cells, 49 / 28 / 33.7 G at 5.8 M, 57.7 / 41.0 / 46.7 G at 105 M (CPML all
+// round); four field sets of 5.8 M cells 55 / 37 / 44 G.
 #include "direct.cuh"
 #include "lumped.cuh"
 
@@ -133,8 +134,9 @@ __device__ __forceinline__ T alpha_of(const Vec<T, V>& a, T b, float a0, int c) 
 // The roundings of the update, spelled out: which product of a sum of two the
 // compiler contracts into the FMA depends on the code around it.  These are
 // the ones the stream kernels compile to (Ex: fma(beta, curl, alpha E), the
-// other components fma(alpha, f, +-beta curl)), so both forms, a cell at a
-// time or 16 bytes, give the same bits.
+// other components fma(alpha, f, +-beta curl)), so a cell at a time and 16 bytes
+// give the same bits, and the stream kernels' bits wherever no two slabs of an
+// axis overlap (cell_psi takes all near faces before the far ones there).
 __device__ __forceinline__ float fma_(float a, float b, float c) { return __fmaf_rn(a, b, c); }
 __device__ __forceinline__ double fma_(double a, double b, double c) { return __fma_rn(a, b, c); }
 __device__ __forceinline__ float mul_(float a, float b) { return __fmul_rn(a, b); }
@@ -576,11 +578,15 @@ static void direct_launch(const StencilArgs<T>& a, DirectArgs d, int which, cuda
 }
 
 // Meshes up to this many cells take one cell per thread: their step is the
-// latency of one short thread.  Measured, one cell against 16 bytes per
-// thread (us per step): 7.6 / 9.4 at 10 thousand cells, 8.5 / 11.5 at 100
-// thousand, 12.8 / 13.5 at 262 thousand, 18.5 / 18.3 at 512 thousand; four
-// field sets of 164 thousand cells 24.3 / 20.6.  The cells alone decide, not
-// the batch, so that a field set's bits do not depend on its batch.
+// latency of one short thread.  The line is where one field set with CPML all
+// round crosses (float32 and float64).  Measured, one cell against 16 bytes per
+// thread, us per step with CPML: 7.1 / 9.1 at 11 thousand cells, 8.4 / 9.0 at 101
+// thousand, 10.0 / 10.6 at 148 thousand, 12.1 / 11.3 at 226 thousand; float64
+// 7.4 / 8.3, 9.3 / 9.5, 11.7 / 11.8, 13.8 / 13.7.  Without CPML the two cross at
+// about 50 thousand cells (4.6 / 4.6; 6.0 / 5.4 at 148 thousand), and so do
+// batches in float32 (four sets with CPML 9.1 / 10.5 at 21 thousand, 12.9 / 10.9
+// at 54 thousand, 22.0 / 18.9 at 148 thousand; eight 37.0 / 32.7 there); the rule
+// does not look at either.
 constexpr long long kScalarCells = 150000;
 
 template <typename T>

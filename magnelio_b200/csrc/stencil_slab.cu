@@ -35,9 +35,10 @@
 // flight and returns; the host reads the status after the step.
 //
 // The engine runs these lists where the caller gave a march depth and where
-// many units are dead; elsewhere the direct kernels (stencil.cu) step the
-// same fields to the same bits faster (256^3 with ten CPML layers: 415 us
-// here, 310 us there).
+// they cost less than the direct kernels (slab_on_lists in engine.cu: dead units,
+// large batches clear of CPML, 16-bit coefficients); elsewhere the direct kernels
+// (stencil.cu) step the same fields to the same bits faster (256^3 with ten CPML
+// layers: 400 us here, 315 us there).
 #include "fused_cpml.cuh"
 #include "tile_common.cuh"
 
