@@ -598,8 +598,8 @@ def run_slab(args, world, rank, local):
     return 0
 
 
-SWEEP_CANDIDATES = (("simple", 0, 0), ("stream", 0, 0), ("fused", 7, 0), ("fused", 16, 0), ("fused", 16, 16),
-                    ("fused", 18, 16), ("fused", 19, 16))
+SWEEP_CANDIDATES = (("simple", 0, 0), ("stream", 0, 0), ("fused", 7, 0), ("fused", 16, 0), ("fused", 18, 0),
+                    ("fused", 19, 0), ("fused", 16, 16), ("fused", 18, 16), ("fused", 19, 16))
 
 
 def sweep_point(n: int, args, local: int) -> dict:

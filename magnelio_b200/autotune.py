@@ -43,22 +43,13 @@ DEFAULT_CANDIDATES = (
     ("fused", 8, 0),
     ("fused", 9, 0),
     ("fused", 0, 0),
-    ("fused", 16, 0),  # the slab step's own choice: direct kernels or unit lists
-    # its unit lists
-    ("fused", 16, 16),
-    ("fused", 17, 16),
-    ("fused", 18, 16),
-    ("fused", 19, 16),
-    ("fused", 20, 16),
-    ("fused", 21, 16),
-    ("fused", 22, 16),
-    ("fused", 23, 16),
-    ("fused", 24, 16),
-    ("fused", 25, 16),
+    # the slab step: by its own choice (timed where that is its unit lists), and
+    # on the lists at a depth of 16
+    *(("fused", v, depth) for depth in (0, 16) for v in range(16, 26)),
     ("bulk", 0, 0),
 )
 SLAB_VARIANT_BASE = 16  # fused variants from here on are the slab step
-CANDIDATE_SET = 8  # bump when the candidates change: cached results of another set are not reused
+CANDIDATE_SET = 9  # bump when the candidates change: cached results of another set are not reused
 
 
 @dataclass

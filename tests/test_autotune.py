@@ -122,10 +122,15 @@ def test_the_same_kernels_are_timed_once():
     assert [r[:3] for r in table] == [("fused", 16, 0), ("fused", 16, 16)] and best[:2] == ("fused", 16)
 
 
-def test_every_default_candidate_runs_kernels_of_its_own():
+def test_the_slab_step_is_tuned_on_its_unit_lists_too():
     slabs = [c for c in autotune.DEFAULT_CANDIDATES if c[0] == "fused" and c[1] >= autotune.SLAB_VARIANT_BASE]
-    assert [c for c in slabs if c[2] == 0] == [("fused", 16, 0)]
-    assert {c[1] for c in slabs if c[2] > 0} == set(range(16, 26))  # the unit lists are tuned
+    for depth in (0, 16):
+        assert {c[1] for c in slabs if c[2] == depth} == set(range(16, 26))
+    # without dead units every form of depth 0 is the direct kernels: one of them is timed
+    times = {c: 1.0 for c in autotune.DEFAULT_CANDIDATES}
+    _, table = autotune.tune_engine(SlabEngine(times), autotune.DEFAULT_CANDIDATES)
+    assert not [r for r in table if r[0] == "fused" and r[1] >= autotune.SLAB_VARIANT_BASE and r[2] == 0]
+    assert len({r[:3] for r in table}) == len(table)
 
 
 def test_sixteen_bit_coefficients_are_tuned_against_the_handle_as_it_comes(tmp_path, monkeypatch):
